@@ -180,6 +180,22 @@ struct Transfer {
   std::vector<double> h_val;
 };
 
+// A scalar level as the cluster kernel reads it (mg_cluster.cu): positions are the nodes in
+// colour order, padded to whole warps; a step deals one round of a colour's rows to the row
+// groups of `act` CTAs
+struct CluTable {
+  bool ok = false;
+  int act = 1, steps = 0, Np = 0, entries = 0;  // CTAs, steps of a sweep, positions, most entries of a
+                                                // CTA (0: too many for its shared memory)
+  DBuf<int4> mem;    // the tables below, behind one another
+  const int4 *tab = nullptr;   // [act][steps][groups] {position or -1, first entry, entries, diagonal - first}
+  const int *first = nullptr;  // [act][steps][groups] first of the row's entries in the CTA's copy
+  const int2 *ent = nullptr;   // [act][entries] the copy's entries: {entry of the matrix, position of its column}
+  const int2 *step = nullptr;  // {positions of the colour, 1: last step of it, 2: first step of it}
+  const int *node = nullptr;   // [Np] node at each position, -1 padding
+  const int *col = nullptr;    // [nqq] position of each entry's column
+};
+
 struct SysLevel {
   int N = 0, NL = 0, ndof = 0, nel = 0;
   long nqq = 0, nql = 0, nqqL = 0, nllL = 0, nnz = 0;
@@ -194,6 +210,8 @@ struct SysLevel {
   std::vector<int> col_off;    // [ncolour+1]
   DBuf<int> col_items;
   DBuf<int> item_colour;
+  CluTable clu;          // scalar systems: tables of the cluster kernel
+  DBuf<int4> gsrow;      // scalar systems: {node, first entry, entries, diagonal - first} in colour order
   // Vanka: velocity nodes of the stars of each colour's patches, patch by patch; entry
   // g of vrows is the (patch, star node) pair g, so per-entry data is stored compactly
   std::vector<int> vrow_off;   // [ncolour+1]
@@ -410,6 +428,11 @@ template <class T>
 int prolong_add(exf_sys *s, int lev_f, const T *x_c, T *x_f, double damp);
 template <class T>
 int smooth(exf_sys *s, int lev, const exf_mg_params *p, int nsweeps, T *x, const T *b);
+// levels hi .. 0 of a scalar system's V-cycle in one cluster launch (mg_cluster.cu)
+int build_cluster(exf_sys *s, int lev, const std::vector<int> &items);
+bool mg_cluster_level(const exf_sys *s, int lev, size_t elem);
+template <class T>
+int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi, bool zero_hi);
 // EXF_ERR_CUDA (and clears the flag) when a bounded in-kernel wait ran out since the last call
 int device_wait_status(exf_sys *s);
 // GMRES + ILU level solver (ilu_gmres.cu)

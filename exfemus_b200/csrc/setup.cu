@@ -393,6 +393,14 @@ static int colour_general(exf_sys *s, int l, int nitem, std::vector<int> &col) {
   return colour_items_greedy(m, nitem, order, cptr, cidx, col);
 }
 
+// the rows of a scalar level in colour order
+__global__ void k_gs_rows(const int *items, int N, const int *qq_ptr, const int *diag, int4 *rows) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= N) return;
+  const int n = items[t], k0 = qq_ptr[n];
+  rows[t] = make_int4(n, k0, qq_ptr[n + 1] - k0, diag[n] - k0);
+}
+
 int build_colours(exf_sys *s) {
   exf_mesh *m = s->mesh;
   cudaStream_t st = s->stream;
@@ -420,6 +428,12 @@ int build_colours(exf_sys *s) {
     for (int i = 0; i < nitem; i++) items[pos[col[i]]++] = i;
     EXF_TRY(L.col_items.alloc(nitem));
     EXF_CUDA(cudaMemcpyAsync(L.col_items.p, items.data(), nitem * sizeof(int), cudaMemcpyHostToDevice, st));
+    if (s->nv1 == 0) {
+      EXF_TRY(L.gsrow.alloc(nitem));
+      k_gs_rows<<<nblk(nitem, 256), 256, 0, st>>>(L.col_items.p, nitem, L.qq_ptr.p, L.diag_pos.p, L.gsrow.p);
+      EXF_LAUNCH_CHECK();
+      EXF_TRY(build_cluster(s, l, items));
+    }
     EXF_CUDA(cudaStreamSynchronize(st));
     if (s->kind == EXF_KIND_NS) {
       // star rows of every colour: the velocity nodes of pressure row m (qq(m)), patch by

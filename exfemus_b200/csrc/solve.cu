@@ -17,6 +17,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "cluster.cuh"
 #include "exf_internal.h"
 
 namespace exf {
@@ -358,22 +359,43 @@ template int prolong_cond<float>(exf_sys *, int, const float *, float *, double,
 // ------------------------------------------------------ Gauss-Seidel (scalar)
 // one colour: nodes of one colour never share an element, so they are not coupled and
 // the colour is updated in parallel exactly as a sequential sweep would.
-template <class T, int LPR>
-__global__ void k_gs_colour(const int *__restrict__ items, int nitems, const int *__restrict__ qq_ptr,
-                            const int *__restrict__ qq_col, const int *__restrict__ diag_pos,
-                            const T *__restrict__ vv, const T *__restrict__ b, T *x) {
-  EXF_PDL_WAIT();
+// What bounds a colour is its chain of dependent loads, not its data: everything that a
+// sweep does not change (descriptor, columns, values, diagonal) is loaded before the wait
+// for the previous colour, so only the gathers of x follow it.  E entries per lane are held
+// in registers; longer rows take the loop behind them.
+template <class T, int LPR, int E>
+__global__ void __launch_bounds__(256) k_gs_colour(const int4 *__restrict__ rows, int nrows,
+                                                   const int *__restrict__ col, const T *__restrict__ vv,
+                                                   const T *__restrict__ b, T *x) {
   const int lane = threadIdx.x % LPR;
   const long g = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
-  const bool valid = g < nitems;  // all lanes reach the shuffles
-  const int n = valid ? items[g] : 0;
-  const int dp = valid ? diag_pos[n] : 0;
-  T acc[1] = {T(0)};
-  if (valid) node_row_dot<T, 1, LPR, false>(n, lane, 0, qq_ptr, qq_col, nullptr, nullptr, 0, 0, vv, nullptr, x, acc);
+  int4 q = make_int4(-1, 0, 0, 0);
+  if (g < nrows) q = rows[g];
+  int c[E];
+  T v[E], diag = T(1);
 #pragma unroll
-  for (int o = LPR / 2; o > 0; o >>= 1) acc[0] += __shfl_down_sync(0xffffffffu, acc[0], o, LPR);
-  // the row product included the diagonal term; remove it (x[n] is not updated yet)
-  if (valid && lane == 0) x[n] = (b[n] - (acc[0] - vv[dp] * x[n])) / vv[dp];
+  for (int e = 0; e < E; e++) {
+    const int i = e * LPR + lane;
+    c[e] = -1;
+    if (i < q.z && i != q.w) {
+      c[e] = col[q.y + i];
+      v[e] = vv[q.y + i];
+    }
+  }
+  if (q.x >= 0) diag = vv[q.y + q.w];
+  EXF_PDL_WAIT();
+  const T bv = q.x >= 0 ? b[q.x] : T(0);
+  T xv[E], acc = T(0);
+#pragma unroll
+  for (int e = 0; e < E; e++) xv[e] = c[e] >= 0 ? x[c[e]] : T(0);
+#pragma unroll
+  for (int e = 0; e < E; e++)
+    if (c[e] >= 0) acc += v[e] * xv[e];
+  for (int i = E * LPR + lane; i < q.z; i += LPR)
+    if (i != q.w) acc += vv[q.y + i] * x[col[q.y + i]];
+#pragma unroll
+  for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, LPR);
+  if (q.x >= 0 && lane == 0) x[q.x] = (bv - acc) / diag;
 }
 
 // --------------------------------------------------------------- Vanka
@@ -1346,34 +1368,6 @@ __global__ void k_vanka_apply(const int *__restrict__ vrows, int nr, long gbase,
 // blocks and couplings of its row in the same order as the ROWS kernel, so both give the
 // same sums.  Every wait is bounded: a wait that runs out sets the system's wait flag and
 // the kernel leaves once its copies have landed.
-#ifndef EXF_WAIT_TRIES
-#define EXF_WAIT_TRIES (1 << 22)
-#endif
-
-__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t *b, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_tx(uint64_t *b, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *b) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
-}
-// true once the phase of parity `par` has completed; false after `tries` tries
-__device__ __forceinline__ bool mbar_wait(uint64_t *b, unsigned par, int tries = EXF_WAIT_TRIES) {
-  for (int t = 0; t < tries; t++) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_addr(b)), "r"(par)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, uint64_t *bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                    smem_addr(dst)),
@@ -2047,13 +2041,18 @@ int vanka_prep(exf_sys *s, int lev) {
 template <class T>
 static int gs_sweep(exf_sys *s, int lev, const exf_mg_params *p, T *x, const T *b) {
   SysLevel &L = s->L[lev];
-  constexpr int LPR = 16;
+  // lanes per row and entries per lane cover the meshes' rows (2D at most 25 entries, 3D 125);
+  // top level of the 513 x 513 lattice, FP64: 46 us per sweep with the loads behind the wait,
+  // 36 us now; the 129 x 33 x 33 lattice 182 us, now 114 us (32 lanes x 4: 112 us, but
+  // slower on its small levels)
+  const int lpr = s->dim == 2 ? 8 : 16;
+  auto kern = s->dim == 2 ? k_gs_colour<T, 8, 4> : k_gs_colour<T, 16, 8>;
   for (int cc = 0; cc < L.ncolour; cc++) {
     const int c = p->reverse_colours ? L.ncolour - 1 - cc : cc;
     const int n = L.col_off[c + 1] - L.col_off[c];
     if (n == 0) continue;
-    EXF_CUDA(launch_pdl(k_gs_colour<T, LPR>, dim3(nblk((long)n * LPR, 256)), dim3(256), 0, s->stream,
-                        L.col_items.p + L.col_off[c], n, L.qq_ptr.p, L.qq_col.p, L.diag_pos.p, VT<T>::vv(L), b, x));
+    EXF_CUDA(launch_pdl(kern, dim3(nblk((long)n * lpr, 256)), dim3(256), 0, s->stream, L.gsrow.p + L.col_off[c], n,
+                        L.qq_col.p, VT<T>::vv(L), b, x));
     EXF_COUNT(1);
   }
   return EXF_OK;
