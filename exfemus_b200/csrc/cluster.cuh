@@ -60,6 +60,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *b, unsigned par, int tries =
   return false;
 }
 
+// bulk copy into this CTA's shared memory, completing on its mbarrier (16-byte aligned)
+__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, uint64_t *bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_addr(dst)),
+               "l"(src), "r"(bytes), "r"(smem_addr(bar))
+               : "memory");
+}
+
 // asynchronous store of two or four consecutive values into the shared memory of a CTA of the
 // cluster, completing on an mbarrier of the same CTA: the receiver waits for the data
 // themselves, no barrier or fence is needed.  `addr` is aligned to the stored vector.

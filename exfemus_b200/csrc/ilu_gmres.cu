@@ -36,6 +36,7 @@
 #include <cmath>
 #include <vector>
 
+#include "cluster.cuh"
 #include "exf_internal.h"
 
 namespace exf {
@@ -203,28 +204,29 @@ __global__ void __launch_bounds__(32 * NW) k_ilu_factor(int N, const int *__rest
       lk[u] = k < last ? Lat(last, k) : 0.;
       uk[u] = k < last ? Lat(k, last) : 0.;
     }
-    for (int j = 0; j < last; j++) {  // L[last][k] -= L[last][j] * L[j][k] / L[j][j]
-      const double lj = __shfl_sync(0xffffffffu, pick(lk, j >> 5), j & 31), djj = Lat(j, j);
-#pragma unroll
-      for (int u = 0; u < KU; u++) {
-        const int k = lane + 32 * u;
-        if (k > j && k < last) lk[u] = __dsub_rn(lk[u], __ddiv_rn(__dmul_rn(lj, Lat(j, k)), djj));
-      }
-    }
-    for (int j = 0; j < last; j++) {  // L[k][last] -= L[j][last] * L[k][j] / L[j][j]
+    // L[last][k] -= L[last][j] * L[j][k] / L[j][j] and, independent of it,
+    // L[k][last] -= L[j][last] * L[k][j] / L[j][j]: the two chains of divisions side by side
+    for (int j = 0; j < last; j++) {
+      const double lj = __shfl_sync(0xffffffffu, pick(lk, j >> 5), j & 31);
       const double uj = __shfl_sync(0xffffffffu, pick(uk, j >> 5), j & 31), djj = Lat(j, j);
 #pragma unroll
       for (int u = 0; u < KU; u++) {
         const int k = lane + 32 * u;
-        if (k > j && k < last) uk[u] = __dsub_rn(uk[u], __ddiv_rn(__dmul_rn(uj, Lat(k, j)), djj));
+        if (k > j && k < last) {
+          lk[u] = __dsub_rn(lk[u], __ddiv_rn(__dmul_rn(lj, Lat(j, k)), djj));
+          uk[u] = __dsub_rn(uk[u], __ddiv_rn(__dmul_rn(uj, Lat(k, j)), djj));
+        }
       }
     }
-    double d = Lat(last, last);  // L[last][last] -= L[j][last] * L[last][j] / L[j][j]
-    for (int j = 0; j < last; j++) {
-      const double uj = __shfl_sync(0xffffffffu, pick(uk, j >> 5), j & 31);
-      const double lj = __shfl_sync(0xffffffffu, pick(lk, j >> 5), j & 31);
-      d = __dsub_rn(d, __ddiv_rn(__dmul_rn(uj, lj), Lat(j, j)));
+    // L[last][last] -= L[j][last] * L[last][j] / L[j][j]: the terms at once, then in order
+    double qd[KU];
+#pragma unroll
+    for (int u = 0; u < KU; u++) {
+      const int k = lane + 32 * u;
+      qd[u] = k < last ? __ddiv_rn(__dmul_rn(uk[u], lk[u]), Lat(k, k)) : 0.;
     }
+    double d = Lat(last, last);
+    for (int j = 0; j < last; j++) d = __dsub_rn(d, __shfl_sync(0xffffffffu, pick(qd, j >> 5), j & 31));
     if (fabs(d) < 10. * DBL_MIN && lane == 0) atomicCAS(ctl + 2, 0, i + 1);  // LASZeroPivotErr
 #pragma unroll
     for (int u = 0; u < KU; u++) {
@@ -242,6 +244,106 @@ __global__ void __launch_bounds__(32 * NW) k_ilu_factor(int N, const int *__rest
     __threadfence();
     __syncwarp();
     if (lane == 0) st_rel(flag + i, gen);
+  }
+}
+
+// The factorisation where every row has at most kFacMax entries up to its diagonal (2D
+// meshes), by one CTA, a dependency level at a time, a warp per row.  The general kernel
+// above pays, per level, the flag round trip through L2 and a gather whose places are
+// searched for: 25 us.  Here the places are found once per system (k_ilu_struct), the
+// entries of a warp's next row are on their way while it eliminates the current one, and
+// a level ends with the CTA's barrier.  Same operations, same order, same bits.
+constexpr int kFacMax = 11, kFacCap = 128, kFacLd = kFacMax + 1;
+
+// row t of the level order: {row, first entry, entries up to the diagonal, diagonal entry};
+// its kFacCap {entry, place in the dense block} and the entries (S_a, i) of the rows in S
+__global__ void k_ilu_struct(int N, const int *__restrict__ ord, const int *__restrict__ ptr,
+                             const int *__restrict__ col, const int *__restrict__ dpos, int4 *row, int2 *ent, int *pos) {
+  const int t = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (t >= N) return;
+  const int i = ord[t], k0 = ptr[i], kd = dpos[i], LD = kd - k0 + 1;
+  if (lane == 0) row[t] = make_int4(i, k0, LD, kd);
+  const int S = lane < LD ? col[k0 + lane] : -1;
+  int2 *out = ent + (long)t * kFacCap;
+  int n = 0;
+  for (int a = 0; a < LD; a++) {
+    const int r = __shfl_sync(0xffffffffu, S, a), rb = ptr[r], re = ptr[r + 1];
+    for (int e0 = rb; e0 < re; e0 += 32) {
+      const int k = e0 + lane, c = k < re ? col[k] : -2;
+      int b = -1;
+      for (int q = 0; q < LD; q++)
+        if (__shfl_sync(0xffffffffu, S, q) == c) b = q;
+      const unsigned m = __ballot_sync(0xffffffffu, b >= 0);
+      if (b >= 0) out[n + __popc(m & ((1u << lane) - 1u))] = make_int2(k, a * kFacLd + b);
+      if (c == i) pos[t * 16 + a] = k;
+      n += __popc(m);
+    }
+  }
+  for (int q = n + lane; q < kFacCap; q += 32) out[q] = make_int2(-1, 0);
+}
+
+__global__ void __launch_bounds__(1024) k_ilu_factor_cta(int nlev, const int *__restrict__ loff,
+                                                         const int4 *__restrict__ row, const int2 *__restrict__ ent,
+                                                         const int *__restrict__ pos, double *f, double *invd, int *ctl) {
+  __shared__ double s_blk[32][kFacMax * kFacLd + 4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double *B = s_blk[warp];
+  int4 rw = make_int4(0, 0, 0, 0);
+  int2 e[4];
+  int pi = 0;
+  auto fetch = [&](int t) {
+    rw = row[t];
+    pi = lane < 16 ? pos[t * 16 + lane] : 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) e[q] = ent[(long)t * kFacCap + 32 * q + lane];
+  };
+  int lo = loff[0], hi = loff[1], hi2 = nlev > 1 ? loff[2] : hi;
+  if (lo + warp < hi) fetch(lo + warp);
+  for (int l = 0; l < nlev; l++) {
+    const int hi3 = l + 3 <= nlev ? loff[l + 3] : hi2;
+    bool have = lo + warp < hi;
+    for (int t = lo + warp; t < hi; t += 32) {
+      double g[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) g[q] = e[q].x >= 0 ? f[e[q].x] : 0.;
+      for (int q = lane; q < kFacMax * kFacLd; q += 32) B[q] = 0.;
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (e[q].x >= 0) B[e[q].y] = g[q];
+      __syncwarp();
+      const int i = rw.x, k0 = rw.y, last = rw.z - 1, kd = rw.w, pk = pi;
+      // the warp's next row, of this level or the next
+      const int tn = t + 32 < hi ? t + 32 : hi + warp;
+      if (tn < (t + 32 < hi ? hi : hi2)) fetch(tn);
+      double lk = lane < last ? B[last * kFacLd + lane] : 0., uk = lane < last ? B[lane * kFacLd + last] : 0.;
+      for (int j = 0; j < last; j++) {
+        const double lj = __shfl_sync(0xffffffffu, lk, j), uj = __shfl_sync(0xffffffffu, uk, j);
+        const double djj = B[j * kFacLd + j];
+        if (lane > j && lane < last) {
+          lk = __dsub_rn(lk, __ddiv_rn(__dmul_rn(lj, B[j * kFacLd + lane]), djj));
+          uk = __dsub_rn(uk, __ddiv_rn(__dmul_rn(uj, B[lane * kFacLd + j]), djj));
+        }
+      }
+      const double qd = lane < last ? __ddiv_rn(__dmul_rn(uk, lk), B[lane * kFacLd + lane]) : 0.;
+      double d = B[last * kFacLd + last];
+      for (int j = 0; j < last; j++) d = __dsub_rn(d, __shfl_sync(0xffffffffu, qd, j));
+      if (fabs(d) < 10. * DBL_MIN && lane == 0) atomicCAS(ctl + 2, 0, i + 1);  // LASZeroPivotErr
+      if (lane < last) {
+        f[k0 + lane] = lk;
+        f[pk] = uk;
+      }
+      if (lane == 0) {
+        f[kd] = d;
+        invd[i] = __ddiv_rn(1., d);
+      }
+      __syncwarp();
+    }
+    if (!have && hi + warp < hi2) fetch(hi + warp);
+    lo = hi;
+    hi = hi2;
+    hi2 = hi3;
+    __syncthreads();
   }
 }
 
@@ -311,6 +413,183 @@ __global__ void __launch_bounds__(128) k_ilu_upper(int N, const int *__restrict_
   }
 }
 
+
+// ILUPrecond of a level whose vector fits one CTA's shared memory: both triangular solves in
+// one launch of one CTA, dependency level after dependency level.  What bounds a solve is
+// the round trip from a row's value to the rows that read it, once per level: 3 us through
+// L2 between warps (the kernels above).  Here a few warps solve in turn, a thread per row,
+// doing the reference's operations in the reference's order, and the values stay in shared
+// memory.  Their instructions are then the bound, so the factor comes as a stream in the order of its
+// use (another warp copies it into shared-memory stages): records of up to 32 rows of one
+// level and up to kTriE entries of each, in planes of 32 (constant strides):
+//   {groups of 4 entries, 1: first of its rows | 2: last | 4: last of its chunk, 16-byte
+//   words, 0}, row[32],
+//   1 / d [32], d[32], index[entries][32], value[entries][32]
+// A row of more entries continues in the next record.  Absent entries and rows point to a
+// zero behind the vector (s - 0 * 0 leaves the bits of s).  v holds c, then
+// w = (D + L)^-1 c, then y, in place: a row reads its own c (w) before it replaces it.
+constexpr int kTriE = 24, kTriStages = 4, kTriThreads = 256, kTriWarps = 4;
+constexpr int tri_words(int M) { return 41 + 24 * M; }  // M: a multiple of 4
+constexpr int kTriWords = 2 * tri_words(kTriE);  // a stage: two records at least
+constexpr size_t kTriSmem = 224 * 1024;
+
+struct TriSmem {
+  uint4 st[kTriStages][kTriWords];
+  uint64_t full[kTriStages], empty[kTriStages], turn[kTriWarps];
+  double part[32];        // sums of rows that continue in the next record
+  int words[kTriStages];  // of the chunk in each stage
+};
+struct TriRow {  // a lane's row of a record, loaded a record ahead
+  int g, flags, i;
+  double inv, dia;
+  int c[kTriE];
+  double a[kTriE];
+};
+__device__ __forceinline__ void tri_load(TriRow &t, const uint4 *rec, const uint4 h, int lane) {
+  t.g = (int)h.x;
+  t.flags = (int)h.y;
+  const int *q = reinterpret_cast<const int *>(rec + 1) + lane;
+  const double *d = reinterpret_cast<const double *>(rec + 9) + lane;
+  const int *col = reinterpret_cast<const int *>(rec + 41) + lane;
+  const double *val = reinterpret_cast<const double *>(rec + 41 + 32 * t.g) + lane;
+  t.i = q[0];
+  t.inv = d[0];
+  t.dia = d[32];
+#pragma unroll
+  for (int g = 0; g < kTriE / 4; g++)
+    if (g < t.g) {
+#pragma unroll
+      for (int u = 4 * g; u < 4 * g + 4; u++) {
+        t.c[u] = col[u * 32];
+        t.a[u] = val[u * 32];
+      }
+    }
+}
+__device__ __forceinline__ void tri_solve(const TriRow &t, double *v, double *part, int lane, bool upper) {
+  double s = t.flags & 1 ? 0. : part[lane];
+  const double w = v[t.i];
+  double x[kTriE];
+#pragma unroll
+  for (int g = 0; g < kTriE / 4; g++)  // every gather before the first product
+    if (g < t.g) {
+#pragma unroll
+      for (int u = 4 * g; u < 4 * g + 4; u++) x[u] = v[t.c[u]];
+    }
+#pragma unroll
+  for (int g = 0; g < kTriE / 4; g++)
+    if (g < t.g) {
+      double p[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) p[u] = __dmul_rn(t.a[4 * g + u], x[4 * g + u]);
+#pragma unroll
+      for (int u = 0; u < 4; u++) s = __dsub_rn(s, p[u]);
+    }
+  if (t.flags & 2)  // lower: (Sum + c_i) / d; upper: (Sum + (0 + d_i w_i)) / d
+    v[t.i] = __dmul_rn(__dadd_rn(s, upper ? __dadd_rn(0., __dmul_rn(t.dia, w)) : w), t.inv);
+  else part[lane] = s;
+}
+
+__global__ void __launch_bounds__(kTriThreads) k_ilu_tri(int N, const uint4 *__restrict__ str,
+                                                         const int2 *__restrict__ chunk, int nch, int nlo, int nrec,
+                                                         const double *c, double *y, int *err, const int *skip) {
+  if (skip && *skip) return;
+  extern __shared__ __align__(16) unsigned char tri_raw[];
+  TriSmem &S = *reinterpret_cast<TriSmem *>(tri_raw);
+  double *v = reinterpret_cast<double *>(tri_raw + sizeof(TriSmem));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
+    for (int k = 0; k < kTriStages; k++) {
+      mbar_init(&S.full[k], 1);
+      mbar_init(&S.empty[k], 1);
+    }
+    for (int k = 0; k < kTriWarps; k++) mbar_init(&S.turn[k], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    v[N] = 0.;
+  }
+#pragma unroll 4
+  for (int i = tid; i < N; i += kTriThreads) v[i] = c[i];
+  __syncthreads();
+  if (tid == 32 * kTriWarps) {  // producer: chunk after chunk
+    int it = 0;
+    bool ok = true;
+    int2 ch = chunk[0];
+    for (; it < nch; it++) {
+      const int k = it % kTriStages;
+      if (it >= kTriStages && !mbar_wait(&S.empty[k], ((it / kTriStages) - 1) & 1)) {
+        ok = false;
+        break;
+      }
+      S.words[k] = ch.y;
+      mbar_arrive_tx(&S.full[k], (unsigned)ch.y * 16u);
+      bulk_g2s(&S.st[k][0], str + ch.x, (unsigned)ch.y * 16u, &S.full[k]);
+      if (it + 1 < nch) ch = chunk[it + 1];
+    }
+    if (!ok) {  // the copies already issued land before the CTA leaves
+      atomicExch(err, 1);
+      for (int j = max(0, it - kTriStages); j < it; j++) mbar_wait(&S.full[j % kTriStages], (j / kTriStages) & 1);
+    }
+  } else if (warp < kTriWarps) {
+    // the warps solve the records in turn; while one solves, the others load their next
+    int it = -1, o = 0, words = 0;  // the newest chunk looked at, the place of its next record
+    bool good = true;
+    auto next_record = [&](uint4 &h) -> const uint4 * {  // nullptr after a wait that ran out
+      if (o >= words && good) {
+        it++;
+        const int k = it % kTriStages;
+        if (!mbar_wait(&S.full[k], (it / kTriStages) & 1)) {
+          atomicExch(err, 1);
+          good = false;
+        }
+        o = 0;
+        words = S.words[k];
+      }
+      if (!good) return nullptr;
+      const uint4 *r = &S.st[it % kTriStages][o];
+      h = r[0];
+      o += (int)h.z;
+      return r;
+    };
+    TriRow t;
+    int ci = 0;  // chunk of the record in hand
+    bool have = false;
+    auto fetch = [&](int skip) {
+      uint4 h;
+      for (int q = 0; q < skip; q++) next_record(h);
+      const uint4 *r = next_record(h);
+      have = r != nullptr;
+      ci = it;
+      if (have) tri_load(t, r, h, lane);
+    };
+    if (warp < nrec) fetch(warp);
+    for (int k = warp, turn = warp == 0 ? -1 : 0; k < nrec; k += kTriWarps, turn++) {
+      if (turn >= 0 && !mbar_wait(&S.turn[warp], turn & 1)) {  // record k - 1 is solved
+        atomicExch(err, 1);
+        good = have = false;  // the turns go on without further work
+      }
+      if (have) tri_solve(t, v, S.part, lane, k >= nlo);
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&S.turn[(warp + 1) % kTriWarps]);
+        // the last record of a chunk (all its others are solved) frees the chunk's stage
+        if (have && (t.flags & 4)) mbar_arrive(&S.empty[ci % kTriStages]);
+      }
+      have = false;
+      if (k + kTriWarps < nrec) fetch(kTriWarps - 1);
+    }
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int i = tid; i < N; i += kTriThreads) y[i] = v[i];
+}
+
+// the factor's values into the streams: {double of the stream, entry of f or ~row of 1 / d}
+__global__ void k_ilu_stream(const int2 *__restrict__ src, int n, const double *__restrict__ f,
+                             const double *__restrict__ invd, double *__restrict__ str) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int2 e = src[i];
+  str[e.x] = e.y >= 0 ? f[e.y] : invd[~e.y];
+}
 
 // ------------------------------------------------------------------- GMRES scalars
 // gm_sc: [0] ||b||^2, [1] ||v1||^2 (the residual), [2] the last inner product, [4] the
@@ -384,8 +663,7 @@ __global__ void k_gm_axpy(double *v, const double *__restrict__ vk, long n, cons
 
 // h[i][i+1] = ||v_{i+1}|| (the last inner product), then the Q-R update of column i and
 // of s (itersolv.c, the "Q-R algorithm" block)
-__global__ void k_gm_qr(double *sc, int i) {
-  const double nrm = __dsqrt_rn(sc[2]);
+__device__ __forceinline__ void gm_qr_column(double *sc, int i, double nrm) {
   sc[gmH(i, i + 1)] = nrm;
   sc[4] = nrm;
   for (int k = 1; k < i; k++) {
@@ -404,6 +682,7 @@ __global__ void k_gm_qr(double *sc, int i) {
   sc[gmS(i + 1)] = __dmul_rn(-sc[gmC2(i)], sc[gmS(i)]);
   sc[gmS(i)] = __dmul_rn(sc[gmC1(i)], sc[gmS(i)]);
 }
+__global__ void k_gm_qr(double *sc, int i) { gm_qr_column(sc, i, __dsqrt_rn(sc[2])); }
 
 // H y = s by back substitution (s is overwritten, as in the reference)
 __global__ void k_gm_solve(double *sc, int ni) {
@@ -425,6 +704,68 @@ __global__ void k_gm_update(double *x, const double *__restrict__ V, long n, int
 }
 __global__ void k_gm_copy(const double *src, double *dst) { *dst = *src; }
 
+// The same steps for a vector that fits one CTA's shared memory: an Arnoldi step is 3 i + 5
+// launches of 2-3 us above, whatever the size, and one launch here.
+constexpr int kGmCta = 1024;
+constexpr size_t kGmSmem = 200 * 1024;
+
+// block sum, the same value in every thread
+__device__ __forceinline__ double gm_sum(double v, double *sh) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();  // sh is free again
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = sh[threadIdx.x & 31];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// ||b||^2 and the relative-residual test of a call's start
+__global__ void __launch_bounds__(kGmCta) k_gm_begin(const double *__restrict__ b, int n, double *sc, int *ctl,
+                                                     double eps) {
+  __shared__ double sh[kGmCta / 32];
+  double v = 0.;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += kGmCta) v += b[i] * b[i];
+  v = gm_sum(v, sh);
+  if (threadIdx.x > 0) return;
+  sc[0] = v;
+  const double rn = sqrt(sc[1]), bn = sqrt(v);
+  const bool conv = rn < eps * bn || (fabs(bn) < 10. * DBL_MIN && fabs((1. + rn) - 1.) < 10. * DBL_EPSILON);
+  ctl[0] = conv ? 1 : 0;
+}
+// v[1] to unit length, s[1] its norm (i = 0); or v[i + 1] orthogonalised against v[1 .. i]
+// (modified Gram-Schmidt), the Q-R update of column i, and to unit length
+__global__ void __launch_bounds__(kGmCta) k_gm_step(double *V, int n, int i, double *sc, const int *skip) {
+  if (*skip) return;
+  extern __shared__ double gm_v[];
+  __shared__ double sh[kGmCta / 32];
+  double *w = V + (long)i * n;
+#pragma unroll 4
+  for (int q = threadIdx.x; q < n; q += kGmCta) gm_v[q] = w[q];
+  for (int k = 1; k <= i; k++) {
+    const double *vk = V + (long)(k - 1) * n;
+    double d = 0.;
+#pragma unroll 4
+    for (int q = threadIdx.x; q < n; q += kGmCta) d += gm_v[q] * vk[q];
+    const double h = gm_sum(d, sh);
+    if (threadIdx.x == 0) sc[gmH(i, k)] = h;
+#pragma unroll 4
+    for (int q = threadIdx.x; q < n; q += kGmCta) gm_v[q] = __dsub_rn(gm_v[q], __dmul_rn(h, vk[q]));
+  }
+  double d = 0.;
+#pragma unroll 4
+  for (int q = threadIdx.x; q < n; q += kGmCta) d += gm_v[q] * gm_v[q];
+  const double nrm = __dsqrt_rn(gm_sum(d, sh)), f = __ddiv_rn(1., nrm);
+#pragma unroll 4
+  for (int q = threadIdx.x; q < n; q += kGmCta) w[q] = __dmul_rn(gm_v[q], f);
+  if (threadIdx.x > 0) return;
+  if (i == 0) {
+    sc[gmS(1)] = nrm;
+  } else {
+    gm_qr_column(sc, i, nrm);
+  }
+}
+
 // ------------------------------------------------------------------- host side
 static int ilu_grid(exf_sys *s) { return s->nsm * 2; }
 
@@ -441,6 +782,13 @@ static int dot_dev(exf_sys *s, SysLevel &L, const double *a, const double *b, lo
 static int ilu_apply_dev(exf_sys *s, int lev, const double *c, double *y, const int *skip) {
   SysLevel &L = s->L[lev];
   const int N = L.N, G = ilu_grid(s);
+  if (L.ilu_nsrc) {  // the streams exist: one CTA
+    k_ilu_tri<<<1, kTriThreads, sizeof(TriSmem) + (size_t)(N + 1) * sizeof(double), s->stream>>>(
+        N, L.ilu_str.p, L.ilu_chunk.p, L.ilu_nchunk, L.ilu_nrec[0], L.ilu_nrec[0] + L.ilu_nrec[1], c, y, s->wait_flag.p, skip);
+    EXF_COUNT(1);
+    EXF_LAUNCH_CHECK();
+    return EXF_OK;
+  }
   const unsigned g = (unsigned)((N + 255) / 256);
   k_ilu_prep<<<g, 256, 0, s->stream>>>(L.gm_w.p, N, L.ilu_ctl.p, skip);
   k_ilu_lower<<<G, 128, 0, s->stream>>>(N, L.ilu_ord_lo.p, L.qq_ptr.p, L.qq_col.p, L.diag_pos.p, L.ilu_f.p,
@@ -473,7 +821,7 @@ static int launch_factor(exf_sys *s, SysLevel &L) {
 // (consecutive rows of the level-nested numbering mostly depend on each other).
 // Returns the number of levels.
 static int level_order(const std::vector<int> &ptr, const std::vector<int> &col, const std::vector<int> &dp,
-                       bool upper, std::vector<int> &ord) {
+                       bool upper, std::vector<int> &ord, std::vector<int> *level = nullptr) {
   const int N = (int)dp.size();
   std::vector<int> lv(N, 0);
   int nl = 0;
@@ -490,7 +838,73 @@ static int level_order(const std::vector<int> &ptr, const std::vector<int> &col,
   for (int l = 0; l < nl; l++) cnt[l + 1] += cnt[l];
   ord.assign(N, 0);
   for (int i = 0; i < N; i++) ord[cnt[lv[i]]++] = i;
+  if (level) *level = std::move(lv);
   return nl;
+}
+
+// The streams of k_ilu_tri for one level, from the pattern (fixed per system): the rows by
+// dependency level, a level's rows longest first, consecutive records packed into chunks
+static int build_streams(exf_sys *s, SysLevel &L, const std::vector<int> &ptr, const std::vector<int> &col,
+                         const std::vector<int> &dp) {
+  const int N = L.N;
+  if (sizeof(TriSmem) + (size_t)(N + 1) * sizeof(double) > kTriSmem) return EXF_OK;
+  EXF_CUDA(cudaFuncSetAttribute(k_ilu_tri, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTriSmem));
+  std::vector<uint4> str;
+  std::vector<int2> src, chunk;
+  size_t newest = 0;  // the last record
+  L.ilu_nrec[0] = L.ilu_nrec[1] = 0;
+  for (int up = 0; up < 2; up++) {
+    std::vector<int> ord, lv;
+    level_order(ptr, col, dp, up == 1, ord, &lv);
+    auto len = [&](int i) { return up ? ptr[i + 1] - 1 - dp[i] : dp[i] - ptr[i]; };
+    for (int a = 0; a < N;) {
+      int e = a;
+      while (e < N && lv[ord[e]] == lv[ord[a]]) e++;
+      std::stable_sort(ord.begin() + a, ord.begin() + e, [&](int x, int y) { return len(x) > len(y); });
+      for (; a < e; a += 32) {
+        const int R = std::min(32, e - a), most = len(ord[a]);
+        for (int j0 = 0; j0 == 0 || j0 < most; j0 += kTriE) {
+          const int M = (std::min(kTriE, most - j0) + 3) & ~3, w = tri_words(M);
+          const size_t o = str.size();
+          if (chunk.empty() || chunk.back().y + w > kTriWords) {
+            if (!chunk.empty()) str[newest].y |= 4u;
+            chunk.push_back(make_int2((int)o, 0));
+          }
+          chunk.back().y += w;
+          newest = o;
+          L.ilu_nrec[up]++;
+          str.resize(o + w, make_uint4(0u, 0u, 0u, 0u));
+          str[o] = make_uint4((unsigned)M / 4, (j0 == 0 ? 1u : 0u) | (j0 + kTriE >= most ? 2u : 0u), (unsigned)w, 0u);
+          int *row = reinterpret_cast<int *>(&str[o + 1]), *ix = reinterpret_cast<int *>(&str[o + 41]);
+          for (int k = 0; k < 32; k++) row[k] = N;
+          for (int k = 0; k < 32 * M; k++) ix[k] = N;
+          for (int r = 0; r < R; r++) {
+            const int i = ord[a + r];
+            row[r] = i;
+            src.push_back(make_int2((int)(2 * (o + 9)) + r, ~i));
+            src.push_back(make_int2((int)(2 * (o + 25)) + r, dp[i]));
+            for (int j = j0; j < std::min(len(i), j0 + M); j++) {
+              const int k = up ? ptr[i + 1] - 1 - j : ptr[i] + j;  // upper: from the row's end
+              ix[(j - j0) * 32 + r] = col[k];
+              src.push_back(make_int2((int)(2 * (o + 41 + 8 * M)) + (j - j0) * 32 + r, k));
+            }
+          }
+        }
+      }
+      a = e;
+    }
+  }
+  str[newest].y |= 4u;
+  L.ilu_nchunk = (int)chunk.size();
+  EXF_TRY(L.ilu_str.alloc(str.size()));
+  EXF_TRY(L.ilu_src.alloc(src.size()));
+  EXF_TRY(L.ilu_chunk.alloc(chunk.size()));
+  EXF_CUDA(cudaMemcpyAsync(L.ilu_str.p, str.data(), str.size() * sizeof(uint4), cudaMemcpyHostToDevice, s->stream));
+  EXF_CUDA(cudaMemcpyAsync(L.ilu_src.p, src.data(), src.size() * sizeof(int2), cudaMemcpyHostToDevice, s->stream));
+  EXF_CUDA(cudaMemcpyAsync(L.ilu_chunk.p, chunk.data(), chunk.size() * sizeof(int2), cudaMemcpyHostToDevice, s->stream));
+  EXF_CUDA(cudaStreamSynchronize(s->stream));
+  L.ilu_nsrc = (int)src.size();
+  return EXF_OK;
 }
 
 // ILUFactor of level lev's matrix, once per assembly (outside graph capture)
@@ -517,14 +931,31 @@ int ilu_ready(exf_sys *s, int lev) {
     EXF_CUDA(cudaStreamSynchronize(s->stream));
     int m = 1;
     for (int i = 0; i < N; i++) m = std::max(m, dp[i] - ptr[i] + 1);
-    std::vector<int> lo, up;
-    L.ilu_depth[0] = level_order(ptr, col, dp, false, lo);
+    std::vector<int> lo, up, lv;
+    L.ilu_depth[0] = level_order(ptr, col, dp, false, lo, &lv);
     L.ilu_depth[1] = level_order(ptr, col, dp, true, up);
     EXF_TRY(L.ilu_ord_lo.alloc(N));
     EXF_TRY(L.ilu_ord_up.alloc(N));
     EXF_CUDA(cudaMemcpyAsync(L.ilu_ord_lo.p, lo.data(), N * sizeof(int), cudaMemcpyHostToDevice, s->stream));
     EXF_CUDA(cudaMemcpyAsync(L.ilu_ord_up.p, up.data(), N * sizeof(int), cudaMemcpyHostToDevice, s->stream));
     EXF_CUDA(cudaStreamSynchronize(s->stream));
+    EXF_TRY(build_streams(s, L, ptr, col, dp));
+    if (m <= kFacMax && N <= (1 << 18)) {
+      std::vector<int> off(L.ilu_depth[0] + 1, 0);
+      for (int i = 0; i < N; i++) off[lv[i] + 1]++;
+      for (int l = 0; l < L.ilu_depth[0]; l++) off[l + 1] += off[l];
+      EXF_TRY(L.ilu_loff.alloc(off.size()));
+      EXF_TRY(L.ilu_ent.alloc((size_t)N * kFacCap));
+      EXF_TRY(L.ilu_pos.alloc((size_t)N * 16));
+      EXF_TRY(L.ilu_row.alloc(N));
+      EXF_TRY(L.ilu_pos.zero(s->stream));
+      EXF_CUDA(cudaMemcpyAsync(L.ilu_loff.p, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
+      EXF_CUDA(cudaStreamSynchronize(s->stream));
+      k_ilu_struct<<<(unsigned)(((long)N * 32 + 255) / 256), 256, 0, s->stream>>>(
+          N, L.ilu_ord_lo.p, L.qq_ptr.p, L.qq_col.p, L.diag_pos.p, L.ilu_row.p, L.ilu_ent.p, L.ilu_pos.p);
+      EXF_COUNT(1);
+      EXF_LAUNCH_CHECK();
+    }
     L.ilu_maxl = m;
     s->buf_epoch++;
   }
@@ -544,10 +975,21 @@ int ilu_ready(exf_sys *s, int lev) {
   }
   EXF_CUDA(cudaMemcpyAsync(L.ilu_f.p, L.A.vv.p, L.nqq * sizeof(double), cudaMemcpyDeviceToDevice, s->stream));
   EXF_CUDA(cudaMemsetAsync(L.ilu_ctl.p + 2, 0, sizeof(int), s->stream));
-  if (L.ilu_maxl <= 16) EXF_TRY((launch_factor<16, 2>(s, L)));
+  if (L.ilu_row.p) {
+    k_ilu_factor_cta<<<1, 1024, 0, s->stream>>>(L.ilu_depth[0], L.ilu_loff.p, L.ilu_row.p, L.ilu_ent.p, L.ilu_pos.p,
+                                                L.ilu_f.p, L.ilu_inv.p, L.ilu_ctl.p);
+    EXF_COUNT(1);
+    EXF_LAUNCH_CHECK();
+  } else if (L.ilu_maxl <= 16) EXF_TRY((launch_factor<16, 2>(s, L)));
   else if (L.ilu_maxl <= 32) EXF_TRY((launch_factor<32, 2>(s, L)));
   else if (L.ilu_maxl <= 64) EXF_TRY((launch_factor<64, 2>(s, L)));
   else EXF_TRY((launch_factor<128, 1>(s, L)));
+  if (L.ilu_nsrc) {
+    k_ilu_stream<<<(L.ilu_nsrc + 255) / 256, 256, 0, s->stream>>>(L.ilu_src.p, L.ilu_nsrc, L.ilu_f.p, L.ilu_inv.p,
+                                                                  reinterpret_cast<double *>(L.ilu_str.p));
+    EXF_COUNT(1);
+    EXF_LAUNCH_CHECK();
+  }
   int zp = 0;
   EXF_CUDA(cudaMemcpyAsync(&zp, L.ilu_ctl.p + 2, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   EXF_CUDA(cudaStreamSynchronize(s->stream));
@@ -595,20 +1037,44 @@ int gmres_smooth(exf_sys *s, int lev, double eps, int m, double *x, const double
   int *ctl = L.gm_ctl.p;
   auto vk = [&](int k) { return V + (long)(k - 1) * n; };  // v[k], 1-based
   const unsigned g = (unsigned)((n + 255) / 256);
-  k_gm_reset<<<1, 1, 0, s->stream>>>(ctl);
-  EXF_TRY(dot_dev(s, L, b, b, n, sc));                                  // bNorm
-  EXF_TRY(spmv_resid<double>(s, lev, x, b, vk(1), sc + 1));             // v[1] = b - A x
+  const bool small = (size_t)n * sizeof(double) <= kGmSmem;  // one CTA per step
+  if (small)
+    EXF_CUDA(cudaFuncSetAttribute(k_gm_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGmSmem));
+  auto step = [&](int i) {
+    k_gm_step<<<1, kGmCta, (size_t)n * sizeof(double), s->stream>>>(V, (int)n, i, sc, ctl);
+    EXF_COUNT(1);
+  };
+  if (small) {
+    EXF_TRY(spmv_resid<double>(s, lev, x, b, vk(1), sc + 1));  // v[1] = b - A x
+    k_gm_begin<<<1, kGmCta, 0, s->stream>>>(b, (int)n, sc, ctl, eps);
+    EXF_COUNT(1);
+  } else {
+    k_gm_reset<<<1, 1, 0, s->stream>>>(ctl);
+    EXF_TRY(dot_dev(s, L, b, b, n, sc));                       // bNorm
+    EXF_TRY(spmv_resid<double>(s, lev, x, b, vk(1), sc + 1));  // v[1] = b - A x
+  }
   for (int iter = 0; iter < m;) {
-    k_gm_rtc<<<1, 1, 0, s->stream>>>(sc, ctl, eps);
+    if (!small || iter > 0) {
+      k_gm_rtc<<<1, 1, 0, s->stream>>>(sc, ctl, eps);
+      EXF_COUNT(1);
+    }
     EXF_TRY(ilu_apply_dev(s, lev, vk(1), vk(1), ctl));
-    EXF_TRY(dot_dev(s, L, vk(1), vk(1), n, sc + 2));
-    k_gm_first<<<1, 1, 0, s->stream>>>(sc);
-    k_gm_scale<<<g, 256, 0, s->stream>>>(vk(1), n, sc + 4, ctl);
-    EXF_COUNT(3);
+    if (small) {
+      step(0);
+    } else {
+      EXF_TRY(dot_dev(s, L, vk(1), vk(1), n, sc + 2));
+      k_gm_first<<<1, 1, 0, s->stream>>>(sc);
+      k_gm_scale<<<g, 256, 0, s->stream>>>(vk(1), n, sc + 4, ctl);
+      EXF_COUNT(2);
+    }
     const int ni = std::min(kGmSteps, m - iter);
     for (int i = 1; i <= ni; i++) {
       EXF_TRY(spmv_resid<double>(s, lev, vk(i), nullptr, L.gm_t.p, nullptr));  // A v[i]
       EXF_TRY(ilu_apply_dev(s, lev, L.gm_t.p, vk(i + 1), ctl));
+      if (small) {
+        step(i);
+        continue;
+      }
       for (int k = 1; k <= i; k++) {  // modified Gram-Schmidt
         EXF_TRY(dot_dev(s, L, vk(i + 1), vk(k), n, sc + gmH(i, k)));
         k_gm_axpy<<<g, 256, 0, s->stream>>>(vk(i + 1), vk(k), n, sc + gmH(i, k), ctl);

@@ -1368,13 +1368,6 @@ __global__ void k_vanka_apply(const int *__restrict__ vrows, int nr, long gbase,
 // blocks and couplings of its row in the same order as the ROWS kernel, so both give the
 // same sums.  Every wait is bounded: a wait that runs out sets the system's wait flag and
 // the kernel leaves once its copies have landed.
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, uint64_t *bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_addr(dst)),
-               "l"(src), "r"(bytes), "r"(smem_addr(bar))
-               : "memory");
-}
-
 static int star_pack(exf_sys *s, int lev);
 
 template <int STG, int CAPB>
