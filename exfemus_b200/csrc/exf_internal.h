@@ -225,6 +225,9 @@ struct SysLevel {
   DBuf<int16_t> tcq, tcl;      // per qq / ql block: column minus row as a 9^d-tile index step
   bool tile_ok = false;        // every star and row fits the tile kernels (5^d nodes)
   DBuf<int> pstart;            // [NL] first vrows entry of each patch (by pressure node)
+  int kmax = 0;                // nodes of the largest star
+  std::vector<int> rest_off;   // [ncolour+1] 2D: nodes outside every star of the colour
+  DBuf<int> rest;
   DBuf<double> vk64, pk64;     // per entry*D: {1/a, D/a, G/a}; per patch: {S, c_mm}
   DBuf<float> vk32, pk32;
   DBuf<double> vres64;         // compact star-row residuals [nvrows*D] + pressure rows [NL]

@@ -516,6 +516,18 @@ int build_colours(exf_sys *s) {
         }
       }
       L.vrow_off[L.ncolour] = (int)rows.size();
+      if (dim == 2 && nitem <= 9 * 4 * s->nsm) {  // small levels: the nodes that a colour leaves as they are
+        std::vector<int> rest, seen(L.N, -1);
+        L.rest_off.assign(L.ncolour + 1, 0);
+        for (int c = 0; c < L.ncolour; c++) {
+          for (int g = L.vrow_off[c]; g < L.vrow_off[c + 1]; g++) seen[rows[g]] = c;
+          for (int n = 0; n < L.N; n++)
+            if (seen[n] != c) rest.push_back(n);
+          L.rest_off[c + 1] = (int)rest.size();
+        }
+        EXF_TRY(L.rest.alloc(rest.size()));
+        EXF_CUDA(cudaMemcpy(L.rest.p, rest.data(), rest.size() * sizeof(int), cudaMemcpyHostToDevice));
+      }
       EXF_TRY(L.vrows.alloc(rows.size()));
       EXF_CUDA(cudaMemcpy(L.vrows.p, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice));
       EXF_TRY(L.pstart.alloc(L.NL));
@@ -543,6 +555,7 @@ int build_colours(exf_sys *s) {
         pin[2 * t + 1] = make_int4(K, lp[mm + 1] - lp[mm], latl(mm, 0) | (latl(mm, 1) << 11) | (latl(mm, 2) << 22), 0);
       }
       const int smax = dim == 3 ? 125 : 25;
+      L.kmax = kmax;
       L.tile_ok = lat && kmax <= smax && rmax <= smax;
       EXF_TRY(L.vrinfo.alloc(vri.size()));
       EXF_CUDA(cudaMemcpy(L.vrinfo.p, vri.data(), vri.size() * sizeof(int4), cudaMemcpyHostToDevice));

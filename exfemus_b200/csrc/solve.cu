@@ -747,6 +747,130 @@ __global__ void __launch_bounds__(NT)
   if (threadIdx.x == 0) x[Lay<I4>::p(m, N, D)] = xp + omega * dp;
 }
 
+// PATCH: the ROWS pair in one launch per colour, for the small levels of 2D systems, whose
+// colours are two launches of 2-2.3 us with next to no data.  One CTA per patch, LPR lanes
+// per star row or pressure row, all of them at once; the residuals go to shared memory and
+// the patch is solved as in k_vanka_solve: the same sums in the same order, so the same bits
+// as ROWS.  The new iterate goes to a second buffer (xn), so no patch of the colour can see
+// another's update; CTAs behind the patches' copy what the colour leaves as it is.  KMAX
+// bounds the star's nodes.
+template <class T, int D, int LPR, int NT, int NTS, int KMAX, bool I4, int UNR, class VB>
+__global__ void __launch_bounds__(NT, 2)
+    k_vanka_patch(const int4 *__restrict__ rinfo, const int4 *__restrict__ pinfo, int npatch, int N, VB vb,
+                  const T *__restrict__ vsc, const int *__restrict__ qq_col, const int *__restrict__ ql_col, long nql,
+                  long nqqL, const T *__restrict__ vp, const T *__restrict__ pv, const T *__restrict__ pp,
+                  const T *__restrict__ vk, const T *__restrict__ pk, const T *__restrict__ x,
+                  const T *__restrict__ b, T *__restrict__ xn, T omega, const int *__restrict__ rest, int nrest,
+                  const int *__restrict__ pcolour, int colour, int NL) {
+  static_assert(NT / LPR > KMAX && KMAX * D <= NTS, "a group per row, a thread per star DOF");
+  __shared__ T s_res[KMAX * D + 1];
+  __shared__ double s_red[NTS / 32];
+  if ((int)blockIdx.x >= npatch) {
+    EXF_PDL_WAIT();
+    const int i = ((int)blockIdx.x - npatch) * NT + threadIdx.x;
+    if (i < nrest) {
+      const int n = rest[i];
+      if constexpr (I4) {
+        reinterpret_cast<float4 *>(xn)[n] = reinterpret_cast<const float4 *>(x)[n];
+      } else {
+#pragma unroll
+        for (int a = 0; a < D; a++) xn[(long)a * N + n] = x[(long)a * N + n];
+      }
+    }
+    if (!I4 && i < NL && pcolour[i] != colour) xn[(long)D * N + i] = x[(long)D * N + i];
+    return;
+  }
+  const int lane = threadIdx.x % LPR;
+  const int4 pi = pinfo[2 * blockIdx.x], pj = pinfo[2 * blockIdx.x + 1];
+  const int m = pi.x, K = pj.x, KD = K * D;
+  const long g0 = pi.y;
+  const PlanarBlocks<T, D> pb{qq_col, pv, nqqL};
+  // what a sweep does not change, before the wait: the group's row (star row r < K, r == K
+  // the pressure row), the solving threads' coefficients and star nodes
+  const int r = threadIdx.x / LPR;
+  int4 q = make_int4(0, 0, 0, 0);
+  if (r < K) q = rinfo[g0 + r];
+  int lc = -1, c[UNR];
+  T lw[D], v[UNR][D * D], sc[D];
+#pragma unroll
+  for (int u = 0; u < UNR; u++) c[u] = -1;
+  if (r < K) {
+#pragma unroll
+    for (int a = 0; a < D; a++) sc[a] = VB::scaled ? vsc[(long)a * N + q.x] : T(1);
+    patch_row_first<T, D, LPR, UNR, D>(lane, q.y, q.w & 0xff, q.z, (q.w >> 8) & 0xff, vb, ql_col, nql, vp, lc, lw, c,
+                                       v);
+  } else if (r == K) {
+    patch_row_first<T, D, LPR, UNR, 1>(lane, pi.z, K, pi.w, pj.y, pb, ql_col, 0, pp, lc, lw, c, v);
+  }
+  const int t = threadIdx.x;
+  const bool solver = t < NTS;
+  T w0 = T(0), w1 = T(0), w2 = T(0);
+  int node = -1;
+  if (t < KD) {
+    const T *w = vk + 3 * (g0 * D + t);
+    w0 = w[0];
+    w1 = w[1];
+    w2 = w[2];
+    node = rinfo[g0 + t / D].x;
+  }
+  const double Sd = (double)pk[2 * m];
+  EXF_PDL_WAIT();
+  T xv = T(0), xp = T(0);
+  if (node >= 0) {
+    xv = x[Lay<I4>::v(t % D, node, N)];
+    // the pressure slots of the star's nodes go along (the patch vertex's is new)
+    if (I4 && t % D == 0 && node != m) xn[Lay<I4>::p(node, N, D)] = x[Lay<I4>::p(node, N, D)];
+  }
+  if (t == 0) xp = x[Lay<I4>::p(m, N, D)];
+  T acc[D], bv[D];
+#pragma unroll
+  for (int a = 0; a < D; a++) acc[a] = bv[a] = T(0);
+  if (r < K) {
+    if (lane == 0) {
+#pragma unroll
+      for (int a = 0; a < D; a++) bv[a] = b[Lay<I4>::v(a, q.x, N)];
+    }
+    patch_row_rest<T, D, LPR, UNR, I4, D>(lane, N, q.y, q.w & 0xff, q.z, (q.w >> 8) & 0xff, vb, ql_col, nql, vp, x,
+                                          acc, sc, lc, lw, c, v);
+  } else if (r == K) {
+    if (lane == 0) bv[0] = b[Lay<I4>::p(m, N, D)];
+    const T one[D] = {};
+    patch_row_rest<T, D, LPR, UNR, I4, 1>(lane, N, pi.z, K, pi.w, pj.y, pb, ql_col, 0, pp, x, acc, one, lc, lw, c, v);
+  }
+#pragma unroll
+  for (int a = 0; a < D; a++)
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) acc[a] += __shfl_down_sync(0xffffffffu, acc[a], o, LPR);
+  if (lane == 0 && r <= K) {
+    const int nv = r < K ? D : 1;
+#pragma unroll
+    for (int a = 0; a < D; a++)
+      if (a < nv) s_res[r * D + a] = bv[a] - acc[a];
+  }
+  __syncthreads();
+  if (solver) {
+    double tsum = node >= 0 ? (double)(w1 * s_res[t]) : 0.;
+    for (int o = 16; o > 0; o >>= 1) tsum += __shfl_down_sync(0xffffffffu, tsum, o);
+    if ((t & 31) == 0) s_red[t >> 5] = tsum;
+  }
+  __syncthreads();
+  if (!solver) return;
+  double Tt = 0.;
+#pragma unroll
+  for (int k = 0; k < NTS / 32; k++) Tt += s_red[k];
+  const double num = Tt - (double)s_res[KD], den = Sd;
+  const T dp = (T)(fabs(den) > 1e-300 ? num / den : 0.);
+  if (node >= 0) xn[Lay<I4>::v(t % D, node, N)] = xv + omega * (s_res[t] * w0 - w2 * dp);
+  if (t == 0) xn[Lay<I4>::p(m, N, D)] = xp + omega * dp;
+}
+
+template <class T>
+__global__ void k_copy(const T *__restrict__ a, T *__restrict__ b, long n) {
+  EXF_PDL_WAIT();
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) b[i] = a[i];
+}
+
 template <class T>
 struct VK;
 template <>
@@ -1886,8 +2010,65 @@ static int vanka_sweep_tile(exf_sys *s, int lev, const exf_mg_params *p, T *x, c
   return EXF_OK;
 }
 
-// AUTO runs the ROWS pair: on the channel, cavity and Boussinesq hierarchies it was
-// measured at least as fast as the tile kernels on every level
+template <class T>
+static const T *vsc_of(const SysLevel &L) {
+  if constexpr (sizeof(T) == 4) return L.vsc.p;
+  else return nullptr;  // FP64 blocks are not scaled
+}
+
+template <class T, class VB>
+static int patch_sweeps(exf_sys *s, SysLevel &L, const exf_mg_params *p, const VB &vb, int nsweeps, T *x, const T *b) {
+  constexpr bool I4 = sizeof(T) == 4;
+  constexpr int KMAX = 25, LPR = 16, NT = LPR * (KMAX + 1), NTS = 64;
+  auto kern = k_vanka_patch<T, 2, LPR, NT, NTS, KMAX, I4, 2, VB>;
+  T *xa = x, *xb = VT<T>::dx(L);
+  for (int it = 0; it < nsweeps; it++)
+    for (int cc = 0; cc < L.ncolour; cc++) {
+      const int c = p->reverse_colours ? L.ncolour - 1 - cc : cc;
+      const int n = L.col_off[c + 1] - L.col_off[c];
+      if (n == 0) continue;
+      const int nrest = L.rest_off[c + 1] - L.rest_off[c];
+      const unsigned ncopy = nblk(std::max(nrest, I4 ? 0 : L.NL), NT);
+      EXF_CUDA(launch_pdl(kern, dim3(n + ncopy), dim3(NT), 0, s->stream, L.vrinfo.p, L.pinfo.p + 2L * L.col_off[c], n,
+                          L.N, vb, vsc_of<T>(L), L.qq_col.p, L.ql_col.p, L.nql, L.nqqL, VT<T>::vp(L), VT<T>::pv(L),
+                          VT<T>::pp(L), VK<T>::vk(L), VK<T>::pk(L), (const T *)xa, b, xb, (T)p->omega,
+                          L.rest.p + L.rest_off[c], nrest, L.item_colour.p, c, L.NL));
+      EXF_COUNT(1);
+      std::swap(xa, xb);
+    }
+  if (xa != x) {  // an odd number of colours: the result is in the second buffer
+    const long len = I4 ? L.len32 : (long)L.ndof;
+    EXF_CUDA(launch_pdl(k_copy<T>, dim3(nblk(len, 256)), dim3(256), 0, s->stream, (const T *)xa, x, len));
+    EXF_COUNT(1);
+  }
+  return EXF_OK;
+}
+
+// AUTO: one launch per colour on 2D levels with at most four patches per SM and colour.  Per
+// sweep, pair against PATCH (FP64 / FP32, us): 17 x 17 nodes 41 / 38 against 25 / 24, 33 x 33
+// 37 / 36 against 27 / 25, 65 x 65 42 / 46 against 28 / 26, 129 x 129 (469 patches a colour)
+// 60 / 48 against 54 / 48; above, the rows of a CTA wait for one another: 257 x 257 159 / 98
+// against 206 / 156
+template <class T>
+static bool patch_level(const exf_sys *s, const SysLevel &L, const exf_mg_params *p) {
+  if (p->vanka_kernel != EXF_VANKA_AUTO || s->dim != 2 || L.kmax > 25 || !L.rest.p) return false;
+  int n = 0;
+  for (int c = 0; c < L.ncolour; c++) n = std::max(n, L.col_off[c + 1] - L.col_off[c]);
+  return n <= 4 * s->nsm;
+}
+template <class T>
+static int vanka_patch(exf_sys *s, int lev, const exf_mg_params *p, int nsweeps, T *x, const T *b) {
+  SysLevel &L = s->L[lev];
+  if constexpr (sizeof(T) == 4) {
+    if (!p->fp32_blocks)
+      return patch_sweeps<T, Packed16<2>>(s, L, p, Packed16<2>{L.qq_col.p, L.h16.p, L.h16cx.p}, nsweeps, x, b);
+  }
+  using VB = PlanarBlocks<T, 4>;
+  return patch_sweeps<T, VB>(s, L, p, VB{L.qq_col.p, VT<T>::vv(L), L.nqq}, nsweeps, x, b);
+}
+
+// AUTO runs the ROWS pair on the other levels: on the channel, cavity and Boussinesq
+// hierarchies it was measured at least as fast as the tile kernels on every level
 template <class T, int D>
 static int vanka_sweep(exf_sys *s, int lev, const exf_mg_params *p, T *x, const T *b) {
   SysLevel &L = s->L[lev];
@@ -2094,6 +2275,7 @@ int smooth(exf_sys *s, int lev, const exf_mg_params *p, int nsweeps, T *x, const
       return EXF_ERR_UNSUPPORTED;
     }
   }
+  if (s->nv1 && patch_level<T>(s, s->L[lev], p)) return vanka_patch<T>(s, lev, p, nsweeps, x, b);
   for (int it = 0; it < nsweeps; it++) {
     if (s->nv1 == 0) {  // scalar systems (T, kappa, omega)
       EXF_TRY(gs_sweep<T>(s, lev, p, x, b));

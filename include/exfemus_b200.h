@@ -78,8 +78,8 @@ extern "C" {
 
 /* Vanka kernel selection (exf_mg_params.vanka_kernel): all compute the same update and
  * differ only in the order of floating-point sums.  AUTO uses BULK on 3D FP32 levels
- * with more than four waves of rows and ROWS elsewhere (each measured fastest there); BULK
- * and ROWS give the same bits. */
+ * with more than four waves of rows, the ROWS pair as one launch per colour on small 2D
+ * levels and ROWS elsewhere (each measured fastest there); all of these give the same bits. */
 #define EXF_VANKA_AUTO 0
 #define EXF_VANKA_TILE 1         /* one CTA per patch, iterate staged in shared memory */
 #define EXF_VANKA_ROWS 2         /* star-row residual kernel + patch-solve kernel      */
