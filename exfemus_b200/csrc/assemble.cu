@@ -185,40 +185,178 @@ __device__ double jac_sur(const FETab<DIM> *t, int q, const double (*xx)[FE<DIM>
   }
 }
 
-// 3D: register cap for 4 CTAs per SM (64 registers, no spills; measured fastest)
-#ifndef EXF_ASM_MINB3
-#define EXF_ASM_MINB3 4
-#endif
-#ifndef EXF_ASM_MINB2
-#define EXF_ASM_MINB2 1
-#endif
+// Launch shape.  3D: CTAs of 128 threads, 4 per SM (the register cap is 128), since an
+// element is a chain of short phases between barriers and only other elements' CTAs fill
+// their latencies.  Whole assembly (k_assemble_levels): NS on the 129 x 33
+// x 33 lattice 2.13 ms at 256 threads and 2 CTAs, 1.92 ms at 128 and 3, 1.86 ms at 128 and
+// 4 (3.06 ms with one pair per thread, 256 and 4, and each phase's loads one after the
+// other); heat 0.91 ms at 256, 0.63 ms at 128 (1.63 ms before).
+constexpr int asm_threads = 128;
+template <int DIM>
+constexpr int asm_ctas = DIM == 2 ? 1 : 4;
+
+template <int N>
+__device__ __forceinline__ void ld16(double (&v)[N], const double *p) {
+  static_assert(N % 2 == 0, "16-byte words");
+  for (int i = 0; i < N / 2; i++) {
+    const double2 w = reinterpret_cast<const double2 *>(p)[i];
+    v[2 * i] = w.x;
+    v[2 * i + 1] = w.y;
+  }
+}
+
+// a matrix entry's read-add-write past L1, as the volume integrals' are
+__device__ __forceinline__ void add_cg(double *p, double v) { __stcg(p, __ldcg(p) + v); }
+
+// The volume integrals of every node pair (i, j) of an element, NB = 1 (T) or DIM * DIM
+// (NS) blocks each, added to the matrix.  With one pair per thread the shared-memory reads
+// (24 values per Gauss point and pair) bound it; in 3D a thread keeps one column j and RI
+// rows i, so a Gauss point's coefficients, column j's shapes and their products are read
+// and formed once for RI pairs.
+//   T (1 accumulator per pair): a warp per row, its lanes the 27 columns, 7 rows a thread:
+//     row reads are broadcasts.  Whole assembly of the 129 x 33 x 33 lattice 0.84 ms with
+//     3 rows and pairs dealt out in thread order, 0.63 ms so.
+//   NS (10 accumulators): 3 rows a thread, pairs in thread order (all lanes busy): 1.86 ms;
+//     4 rows and a warp per row 1.97 ms, 1 row 2.37 ms.
+// The matrix entries are scattered 8-byte words of rows that no other element of this
+// launch touches: prefetched into L2 before the integration (without: NS 2.16 ms against
+// 2.01 ms), read and written past L1, NS row by row so that the old values never sit in
+// registers beside the accumulators.
+template <int DIM, int NT, int NB, int NCO>
+__device__ __forceinline__ void volume_pairs(const AsmArgs<DIM> &A, const int e, const int *s_conn,
+                                             const double (*s_ga)[FE<DIM>::NEN][2],
+                                             const double (*s_gb)[FE<DIM>::NEN][DIM == 3 ? 2 : 1],
+                                             const double (*s_co)[NCO], const int (*s_bcv)[FE<DIM>::NEN]) {
+  using F = FE<DIM>;
+  constexpr int NEN = F::NEN, NQ = F::NQ;
+  constexpr int CA = 1, CL = CA + DIM, CT = CL + DIM;
+  constexpr bool WARP = DIM == 3 && NB == 1;  // a warp per row, its lanes the columns
+  constexpr int RI = DIM == 2 ? 1 : NB == 1 ? 7 : 3;
+  constexpr int ST = WARP ? NT / 32 : NEN / RI;  // rows i0, i0 + ST, ... of a thread
+  constexpr int NP = ST * NEN, NR = WARP ? (NEN + RI * ST - 1) / (RI * ST) : (NP + NT - 1) / NT;
+  static_assert(WARP || NEN % RI == 0, "whole groups of rows");
+#pragma unroll 1
+  for (int r = 0; r < NR; r++) {
+    const int p = threadIdx.x + r * NT;
+    const int j = WARP ? threadIdx.x & 31 : p % NEN;
+    const int i0 = WARP ? r * RI * ST + (threadIdx.x >> 5) : p / NEN;
+    if (WARP ? j >= NEN : p >= NP) break;
+    int blk[RI];
+    for (int m = 0; m < RI; m++) {
+      const int i = min(i0 + m * ST, NEN - 1);  // a row past the last is computed, not stored
+      blk[m] = __ldg(A.qq_ptr + s_conn[i]) + __ldg(A.pos_qq + ((long)e * NEN + i) * NEN + j);
+      for (int c = 0; c < NB; c++)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(&A.vv[(long)c * A.nqq + blk[m]]));
+    }
+    double M[RI], T[RI][NB];
+    for (int m = 0; m < RI; m++) {
+      M[m] = 0.;
+      for (int k = 0; k < NB; k++) T[m][k] = 0.;
+    }
+#pragma unroll 1
+    for (int q = 0; q < NQ; q++) {
+      double co[NCO], pj, gj[DIM];
+      if constexpr (DIM == 3) {
+        double a2[2], b2[2];
+        if constexpr (NB > 1) {
+          ld16(co, s_co[q]);
+        } else {
+          double c8[8];
+          ld16(c8, s_co[q]);
+          for (int k = 0; k < CT; k++) co[k] = c8[k];
+        }
+        ld16(a2, s_ga[q][j]);
+        ld16(b2, s_gb[q][j]);
+        pj = a2[0], gj[0] = a2[1], gj[1] = b2[0], gj[DIM - 1] = b2[1];
+      } else {
+        for (int k = 0; k < (NB > 1 ? NCO : CT); k++) co[k] = s_co[q][k];
+        pj = s_ga[q][j][0], gj[0] = s_ga[q][j][1], gj[1] = s_gb[q][j][0];
+      }
+      double adv = 0., lj[DIM], tj[NB];
+      for (int k = 0; k < DIM; k++) {
+        adv += co[CA + k] * gj[k];
+        lj[k] = co[CL + k] * gj[k];
+      }
+      if constexpr (NB > 1)
+        for (int a = 0; a < DIM; a++)
+          for (int b = 0; b < DIM; b++) tj[a * DIM + b] = co[CT + a * DIM + b] * gj[a];
+      const double mj = co[0] * pj + adv;
+#pragma unroll
+      for (int m = 0; m < RI; m++) {
+        const int i = i0 + m * ST;
+        double pi, gi[DIM], lap = 0.;
+        if constexpr (DIM == 3) {
+          double a2[2], b2[2];
+          ld16(a2, s_ga[q][i]);
+          ld16(b2, s_gb[q][i]);
+          pi = a2[0], gi[0] = a2[1], gi[1] = b2[0], gi[DIM - 1] = b2[1];
+        } else {
+          pi = s_ga[q][i][0], gi[0] = s_ga[q][i][1], gi[1] = s_gb[q][i][0];
+        }
+        for (int k = 0; k < DIM; k++) lap += lj[k] * gi[k];
+        M[m] += pi * mj + lap;
+        if constexpr (NB > 1)
+          for (int a = 0; a < DIM; a++)
+            for (int b = 0; b < DIM; b++) T[m][a * DIM + b] += tj[a * DIM + b] * gi[b];
+      }
+    }
+    constexpr int CH = NB == 1 ? RI : 1;  // rows whose old values are held at a time
+#pragma unroll
+    for (int m0 = 0; m0 < RI; m0 += CH) {
+      double old[CH][NB];
+#pragma unroll
+      for (int m = m0; m < m0 + CH && m < RI; m++)
+        for (int c = 0; c < NB; c++) old[m - m0][c] = __ldcg(A.vv + (long)c * A.nqq + blk[m]);
+#pragma unroll
+      for (int m = m0; m < m0 + CH && m < RI; m++) {
+        const int i = i0 + m * ST;
+        if (i >= NEN) continue;
+        if constexpr (NB == 1) {
+          __stcg(A.vv + blk[m], old[m - m0][0] + s_bcv[0][i] * M[m]);
+        } else {
+          for (int a = 0; a < DIM; a++) {
+            const double bcv = s_bcv[a][i];
+            for (int b = 0; b < DIM; b++) {
+              const double v = T[m][a * DIM + b] + (a == b ? M[m] : 0.);
+              __stcg(A.vv + (long)(a * DIM + b) * A.nqq + blk[m], old[m - m0][a * DIM + b] + bcv * v);
+            }
+          }
+        }
+      }
+    }
+  }
+}
+
 // One element of one level (a CTA): element data, Gauss-point fields and coefficients,
 // the volume integrals of every node pair, B / B^T, the rhs (mode 1) and the boundary
 // sides, each added to the level's matrix in place (elements of one colour share no node).
-template <int DIM, int NT>
+template <int DIM, int NT, bool ns>
 __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const int e, const int mode) {
   using F = FE<DIM>;
   constexpr int NEN = F::NEN, NVX = F::NVX, NQ = F::NQ;
   const int tid = threadIdx.x;
-  const bool ns = A.kind == EXF_KIND_NS;
-  const int nv2 = ns ? DIM : 1;
+  constexpr int nv2 = ns ? DIM : 1;
 
-  __shared__ int s_conn[NEN];
+  __shared__ int s_conn[NEN], s_neigh[F::NSIDE];
   __shared__ double s_xx[DIM][NEN];
   __shared__ int s_bcv[DIM + 1][NEN];
   __shared__ int s_bcb[DIM + 1][NEN];
   __shared__ double s_uold[DIM + 1][NEN];
   __shared__ double s_vold[DIM][NEN];
   __shared__ double s_told[NEN];
-  __shared__ double s_phi[NQ][NEN];
-  __shared__ double s_dphi[NQ][NEN][DIM];
+  // shapes and their derivatives of a node at a Gauss point (the reference element's, then
+  // turned into the global ones in place), read in 16-byte words by the pair integrals:
+  // {phi, d0} in one array, the other derivatives in the next
+  constexpr int GW = DIM == 3 ? 2 : 1;
+  __shared__ __align__(16) double s_ga[NQ + 1][NEN][2];
+  __shared__ __align__(16) double s_gb[NQ + 1][NEN][GW];
   __shared__ double s_psi[NQ][NVX];
   __shared__ double s_ij[NQ][DIM * DIM];
   __shared__ double s_JxW[NQ];
-  __shared__ double s_cM[NQ];          // JxW*rho*inv_dt (NS) or JxW*rhocp*inv_dt (T)
-  __shared__ double s_cA[NQ][DIM];     // JxW*rho*v_k
-  __shared__ double s_cL[NQ][DIM];     // JxW*rho*(nu + f_k v_k^2)
-  __shared__ double s_cT[NQ][DIM * DIM];  // JxW*rho*(nu + f_a v_a v_b)
+  // coefficients of a Gauss point, in this order: JxW*rho*inv_dt (NS) or JxW*rhocp*inv_dt
+  // (T); JxW*rho*v_k; JxW*rho*(nu + f_k v_k^2); JxW*rho*(nu + f_a v_a v_b)
+  constexpr int CA = 1, CL = CA + DIM, CT = CL + DIM, NCO = CT + DIM * DIM;
+  __shared__ __align__(16) double s_co[NQ][NCO];
   __shared__ double s_cR[NQ][DIM];     // rhs coefficient per component
   __shared__ double s_h[DIM];
   __shared__ double s_J[NQ][DIM * DIM];  // Jacobian entries per Gauss point
@@ -226,36 +364,57 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
   __shared__ double s_kt[NEN], s_wt[NEN];  // NS with the eddy viscosity: kappa, omega
 
   const FETab<DIM> *t = A.tab;
-  // ---- element data (get_el_dof_bc, get_el_sol)
+  // ---- element data (get_el_dof_bc, get_el_sol): all of a node's loads in flight before
+  // the first store (A's pointers are generic to the compiler, which keeps every load
+  // behind an earlier shared-memory store: 15 latencies in a row otherwise)
   for (int k = tid; k < NEN; k += NT) {
-    int nd = A.conn[(long)e * NEN + k];
-    s_conn[k] = nd;
-    for (int d = 0; d < DIM; d++) s_xx[d][k] = A.xyz[nd + (long)d * A.ntop];
-    for (int v = 0; v < nv2; v++) {
-      long td = (long)v * A.Ntop + nd;
-      s_bcv[v][k] = A.bc0[td];
-      s_bcb[v][k] = A.bc1[td];
-      s_uold[v][k] = A.xold ? A.xold[td] : 0.;
+    constexpr int NV = ns ? DIM + 1 : 1;
+    const int nd = __ldg(A.conn + (long)e * NEN + k);
+    double xx[DIM], uo[NV], vo[DIM], to = 0., kt = 0., wt = 0.;
+    int bv[NV], bb[NV];
+    for (int d = 0; d < DIM; d++) xx[d] = __ldg(A.xyz + nd + (long)d * A.ntop);
+    for (int v = 0; v < NV; v++) {
+      const bool has = v < nv2 || k < NVX;  // the pressure lives on the vertices
+      const long td = (long)v * A.Ntop + nd;
+      bv[v] = has ? __ldg(A.bc0 + td) : 0;
+      bb[v] = has ? __ldg(A.bc1 + td) : 0;
+      uo[v] = has && A.xold ? __ldg(A.xold + td) : 0.;
     }
-    if (ns && k < NVX) {
-      long td = (long)nv2 * A.Ntop + nd;
-      s_bcv[DIM][k] = A.bc0[td];
-      s_bcb[DIM][k] = A.bc1[td];
-      s_uold[DIM][k] = A.xold ? A.xold[td] : 0.;
-    }
-    for (int d = 0; d < DIM; d++) {
-      if (ns) s_vold[d][k] = s_uold[d][k];
-      else s_vold[d][k] = A.vel ? A.vel[nd + (long)d * A.vel_Ntop] : 0.;
-    }
-    if (ns) s_told[k] = A.temp ? A.temp[nd] : 0.;
-    else s_told[k] = s_uold[0][k];
+    if (!ns)
+      for (int d = 0; d < DIM; d++) vo[d] = A.vel ? __ldg(A.vel + nd + (long)d * A.vel_Ntop) : 0.;
+    if (ns && A.temp) to = __ldg(A.temp + nd);
     if (ns && A.kold) {
-      s_kt[k] = A.kold[nd];
-      s_wt[k] = A.wold[nd];
+      kt = __ldg(A.kold + nd);
+      wt = __ldg(A.wold + nd);
+    }
+    s_conn[k] = nd;
+    for (int d = 0; d < DIM; d++) {
+      s_xx[d][k] = xx[d];
+      s_vold[d][k] = ns ? uo[d < NV ? d : 0] : vo[d];
+    }
+    for (int v = 0; v < NV; v++) {
+      s_bcv[v][k] = bv[v];
+      s_bcb[v][k] = bb[v];
+      s_uold[v][k] = uo[v];
+    }
+    s_told[k] = ns ? to : uo[0];
+    if (ns && A.kold) {
+      s_kt[k] = kt;
+      s_wt[k] = wt;
     }
   }
-  for (int i = tid; i < NQ * NEN; i += NT) (&s_phi[0][0])[i] = (&t->phi[0][0])[i];
-  for (int i = tid; i < NQ * NVX; i += NT) (&s_psi[0][0])[i] = (&t->psi[0][0])[i];
+  if (tid >= 32 && tid < 32 + F::NSIDE) s_neigh[tid - 32] = __ldg(A.neigh + (long)e * F::NSIDE + tid - 32);
+#pragma unroll 2
+  for (int i = tid; i < NQ * NEN; i += NT) {
+    const double ph0 = __ldg(&t->phi[0][0] + i);
+    double dl[DIM];
+    for (int j = 0; j < DIM; j++) dl[j] = __ldg(&t->dphi[0][0][0] + i * DIM + j);
+    (&s_ga[0][0][0])[2 * i] = ph0;
+    (&s_ga[0][0][0])[2 * i + 1] = dl[0];
+    for (int j = 1; j < DIM; j++) (&s_gb[0][0][0])[GW * i + j - 1] = dl[j];
+  }
+#pragma unroll
+  for (int i = tid; i < NQ * NVX; i += NT) (&s_psi[0][0])[i] = __ldg(&t->psi[0][0] + i);
   __syncthreads();
   if (tid < DIM) {
     const int v2 = DIM == 2 ? 2 : 6, v3 = DIM == 2 ? 3 : 7;
@@ -267,27 +426,31 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
   // ---- per Gauss point: Jacobian (src/MGFE.C:1066-1170), fields, coefficients
   const exf_phys &ph = A.ph;
   const double diff_t = ph.inv_prdl * ph.inv_re;
-  const double q_e = (!ns && A.qe) ? A.qe[e] : 0.;
-  // the 27-term sums of every Gauss point first, one per thread (Jacobian entries, then
-  // the interpolated velocity and temperature), each in node order
-  constexpr int NSUM = DIM * DIM + DIM + 1;
-  for (int p = tid; p < NQ * NSUM; p += NT) {
-    const int q = p / NSUM, c = p % NSUM;
-    double sum = 0.;
-    if (c < DIM * DIM) {
-      const int a = c / DIM, b = c % DIM;
-#pragma unroll 1
-      for (int s = 0; s < NEN; s++) sum += s_xx[a][s] * t->dphi[q][s][b];
-      s_J[q][c] = sum;
-    } else if (c < DIM * DIM + DIM) {
-      const int d = c - DIM * DIM;
-#pragma unroll 1
-      for (int k = 0; k < NEN; k++) sum += s_phi[q][k] * s_vold[d][k];
-      s_vg[q][d] = sum;
+  const double q_e = (!ns && A.qe) ? __ldg(A.qe + e) : 0.;
+  // the 27-term sums of every Gauss point first, each in node order: column b of the
+  // Jacobian (b < DIM), or the interpolated velocity and temperature, per thread, so a
+  // shape value is read once for its DIM or DIM + 1 sums
+  for (int p = tid; p < NQ * (DIM + 1); p += NT) {
+    const int b = p / NQ, q = p % NQ;
+    double sum[DIM + 1];
+    for (int c = 0; c <= DIM; c++) sum[c] = 0.;
+    if (b < DIM) {
+      const double *g = b == 0 ? &s_ga[q][0][1] : &s_gb[q][0][b - 1];
+      const int step = b == 0 ? 2 : GW;
+#pragma unroll
+      for (int s = 0; s < NEN; s++) {
+        const double gs = g[s * step];
+        for (int c = 0; c < DIM; c++) sum[c] += s_xx[c][s] * gs;
+      }
+      for (int c = 0; c < DIM; c++) s_J[q][c * DIM + b] = sum[c];
     } else {
-#pragma unroll 1
-      for (int k = 0; k < NEN; k++) sum += s_phi[q][k] * s_told[k];
-      s_vg[q][DIM] = sum;
+#pragma unroll
+      for (int k = 0; k < NEN; k++) {
+        const double f = s_ga[q][k][0];
+        for (int c = 0; c < DIM; c++) sum[c] += f * s_vold[c][k];
+        sum[DIM] += f * s_told[k];
+      }
+      for (int c = 0; c <= DIM; c++) s_vg[q][c] = sum[c];
     }
   }
   __syncthreads();
@@ -321,7 +484,7 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
       inv[o][1] = (J[0][1] * J[o][0] - J[0][0] * J[o][1]) * id;
       inv[o][o] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * id;
     }
-    const double JxW = det * t->w[q];
+    const double JxW = det * __ldg(t->w + q);
     double vg[DIM], mod = 1e-20;
     for (int d = 0; d < DIM; d++) {
       vg[d] = s_vg[q][d];
@@ -333,15 +496,15 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
       for (int i = 0; i < DIM; i++)
         for (int j = 0; j < DIM; j++) s_ij[q][j + i * DIM] = inv[j][i];
       s_JxW[q] = JxW;
-      s_cM[q] = JxW * (ns ? ph.rho : ph.rhocp) * ph.inv_dt;
+      s_co[q][0] = JxW * (ns ? ph.rho : ph.rhocp) * ph.inv_dt;
     }
     const int a = dd;
     if (ns) {
       const double pe = 0.5 * mod * s_h[a] / ph.inv_re;
       const double fa = ph.upwind_ns * ph.rho * 0.5 * (1. / tanh(pe) - 1. / pe) * s_h[a] / mod;
-      s_cA[q][a] = JxW * ph.rho * vg[a];
-      s_cL[q][a] = JxW * ph.rho * (ph.inv_re + fa * vg[a] * vg[a]);
-      for (int b = 0; b < DIM; b++) s_cT[q][a * DIM + b] = JxW * ph.rho * (ph.inv_re + fa * vg[a] * vg[b]);
+      s_co[q][CA + a] = JxW * ph.rho * vg[a];
+      s_co[q][CL + a] = JxW * ph.rho * (ph.inv_re + fa * vg[a] * vg[a]);
+      for (int b = 0; b < DIM; b++) s_co[q][CT + a * DIM + b] = JxW * ph.rho * (ph.inv_re + fa * vg[a] * vg[b]);
       s_cR[q][a] = JxW * (ph.rho * vg[a] * ph.inv_dt + ph.rho * ph.ifr * ph.dirg[a] + ph.buoy * tg * ph.dirg[a]);
     } else {
       double fa = 0.;
@@ -349,19 +512,24 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
         const double pe = 0.5 * mod * s_h[a] / diff_t;
         fa = ph.upwind_t * ph.rhocp * 0.5 * (1. / tanh(pe) - 1. / pe) * s_h[a] / mod;
       }
-      s_cA[q][a] = JxW * ph.rhocp * vg[a];
-      s_cL[q][a] = JxW * (diff_t + fa * vg[a] * vg[a]);
+      s_co[q][CA + a] = JxW * ph.rhocp * vg[a];
+      s_co[q][CL + a] = JxW * (diff_t + fa * vg[a] * vg[a]);
       if (a == 0) s_cR[q][0] = JxW * (ph.rhocp * tg * ph.inv_dt + q_e);
     }
   }
   __syncthreads();
   // global shape derivatives (get_dphi_gl_g, src/MGFE.C:1496-1520)
+#pragma unroll 2
   for (int p = tid; p < NQ * NEN; p += NT) {
     int q = p / NEN, s = p % NEN;
+    double dl[DIM];
+    dl[0] = s_ga[q][s][1];
+    for (int j = 1; j < DIM; j++) dl[j] = s_gb[q][s][j - 1];
     for (int i = 0; i < DIM; i++) {
       double sum = 0.;
-      for (int j = 0; j < DIM; j++) sum += s_ij[q][j + i * DIM] * t->dphi[q][s][j];
-      s_dphi[q][s][i] = sum;
+      for (int j = 0; j < DIM; j++) sum += s_ij[q][j + i * DIM] * dl[j];
+      if (i == 0) s_ga[q][s][1] = sum;
+      else s_gb[q][s][i - 1] = sum;
     }
   }
   __syncthreads();
@@ -375,10 +543,10 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
       for (int a = 0; a < DIM; a++)
         for (int d = 0; d < DIM; d++) g[a][d] = 0.;
       for (int k = 0; k < NEN; k++) {
-        kg += s_phi[q][k] * s_kt[k];
-        wg += s_phi[q][k] * s_wt[k];
+        kg += s_ga[q][k][0] * s_kt[k];
+        wg += s_ga[q][k][0] * s_wt[k];
         for (int a = 0; a < DIM; a++)
-          for (int d = 0; d < DIM; d++) g[a][d] += s_uold[a][k] * s_dphi[q][k][d];
+          for (int d = 0; d < DIM; d++) g[a][d] += s_uold[a][k] * (d == 0 ? s_ga[q][k][1] : s_gb[q][k][d - 1]);
       }
       double sP = 1.e-20;
       for (int a = 0; a < DIM; a++)
@@ -396,8 +564,8 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
       mu_t = fmin(fmax(mu_t, 1.e-6), 1.e+6);
       const double add = s_JxW[q] * ph.rho * IRe * mu_t;
       for (int a = 0; a < DIM; a++) {
-        s_cL[q][a] += add;
-        for (int b = 0; b < DIM; b++) s_cT[q][a * DIM + b] += add;
+        s_co[q][CL + a] += add;
+        for (int b = 0; b < DIM; b++) s_co[q][CT + a * DIM + b] += add;
       }
     }
     __syncthreads();
@@ -405,55 +573,7 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
 
   // ---- volume integrals, node pairs (i,j)
   const int *qq_ptr = A.qq_ptr;
-  for (int p = tid; p < NEN * NEN; p += NT) {
-    const int i = p / NEN, j = p % NEN;
-    const int ni = s_conn[i];
-    const long blk = qq_ptr[ni] + A.pos_qq[((long)e * NEN + i) * NEN + j];
-    if (!ns) {
-      const double old = A.vv[blk];  // loaded before the Gauss-point loop hides its latency
-      double K = 0.;
-#pragma unroll 1
-      for (int q = 0; q < NQ; q++) {
-        const double pi = s_phi[q][i], pj = s_phi[q][j];
-        double adv = 0., lap = 0.;
-        for (int k = 0; k < DIM; k++) {
-          const double gj = s_dphi[q][j][k];
-          adv += s_cA[q][k] * gj;
-          lap += s_cL[q][k] * gj * s_dphi[q][i][k];
-        }
-        K += pi * (s_cM[q] * pj + adv) + lap;
-      }
-      A.vv[blk] = old + s_bcv[0][i] * K;
-    } else {
-      double old[DIM * DIM];  // the pair's entries, loaded before the Gauss-point loop
-      for (int c = 0; c < DIM * DIM; c++) old[c] = A.vv[(long)c * A.nqq + blk];
-      double M = 0., T[DIM * DIM];
-      for (int k = 0; k < DIM * DIM; k++) T[k] = 0.;
-#pragma unroll 1
-      for (int q = 0; q < NQ; q++) {
-        const double pi = s_phi[q][i], pj = s_phi[q][j];
-        double gj[DIM], gi[DIM], adv = 0., lap = 0.;
-        for (int k = 0; k < DIM; k++) {
-          gj[k] = s_dphi[q][j][k];
-          gi[k] = s_dphi[q][i][k];
-          adv += s_cA[q][k] * gj[k];
-          lap += s_cL[q][k] * gj[k] * gi[k];
-        }
-        M += pi * (s_cM[q] * pj + adv) + lap;
-        for (int a = 0; a < DIM; a++) {
-          const double ga = s_dphi[q][j][a];
-          for (int b = 0; b < DIM; b++) T[a * DIM + b] += s_cT[q][a * DIM + b] * ga * gi[b];
-        }
-      }
-      for (int a = 0; a < DIM; a++) {
-        const double bcv = s_bcv[a][i];
-        for (int b = 0; b < DIM; b++) {
-          double v = T[a * DIM + b] + (a == b ? M : 0.);
-          A.vv[(long)(a * DIM + b) * A.nqq + blk] = old[a * DIM + b] + bcv * v;
-        }
-      }
-    }
-  }
+  volume_pairs<DIM, NT, ns ? DIM * DIM : 1, NCO>(A, e, s_conn, s_ga, s_gb, s_co, s_bcv);
   if (ns) {
     // E_b(iv, j) = sum_q JxW psi_iv d_b phi_j : B^T (velocity rows) and B (pressure rows)
     for (int p = tid; p < NVX * NEN; p += NT) {
@@ -461,22 +581,23 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
       // B^T: row (a, node j), column pressure vertex iv; B: pressure row iv, column (b,
       // node j); the entries are loaded before the Gauss-point loop
       const int nj = s_conn[j];
-      const long kq = A.ql_ptr[nj] + A.pos_ql[((long)e * NEN + j) * NVX + iv];
+      const long kq = __ldg(A.ql_ptr + nj) + __ldg(A.pos_ql + ((long)e * NEN + j) * NVX + iv);
       const int niv = s_conn[iv];
-      const long kp = qq_ptr[niv] + A.pos_qq[((long)e * NEN + iv) * NEN + j];
+      const long kp = __ldg(qq_ptr + niv) + __ldg(A.pos_qq + ((long)e * NEN + iv) * NEN + j);
       double oq[DIM], op[DIM];
       for (int a = 0; a < DIM; a++) {
-        oq[a] = A.vp[(long)a * A.nql + kq];
-        op[a] = A.pv[(long)a * A.nqqL + kp];
+        oq[a] = __ldcg(A.vp + (long)a * A.nql + kq);
+        op[a] = __ldcg(A.pv + (long)a * A.nqqL + kp);
       }
       double E[DIM];
       for (int b = 0; b < DIM; b++) E[b] = 0.;
+#pragma unroll 3
       for (int q = 0; q < NQ; q++) {
         const double w = s_JxW[q] * s_psi[q][iv];
-        for (int b = 0; b < DIM; b++) E[b] += w * s_dphi[q][j][b];
+        for (int b = 0; b < DIM; b++) E[b] += w * (b == 0 ? s_ga[q][j][1] : s_gb[q][j][b - 1]);
       }
-      for (int a = 0; a < DIM; a++) A.vp[(long)a * A.nql + kq] = oq[a] + s_bcv[a][j] * (-E[a]);
-      for (int b = 0; b < DIM; b++) A.pv[(long)b * A.nqqL + kp] = op[b] + ph.rho * E[b];
+      for (int a = 0; a < DIM; a++) __stcg(A.vp + (long)a * A.nql + kq, oq[a] + s_bcv[a][j] * (-E[a]));
+      for (int b = 0; b < DIM; b++) __stcg(A.pv + (long)b * A.nqqL + kp, op[b] + ph.rho * E[b]);
     }
   }
   // rhs
@@ -486,7 +607,8 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
       double &r = A.rhs[(long)a * A.N + s_conn[i]];
       const double old = r;
       double F = 0.;
-      for (int q = 0; q < NQ; q++) F += s_phi[q][i] * s_cR[q][a];
+#pragma unroll
+      for (int q = 0; q < NQ; q++) F += s_ga[q][i][0] * s_cR[q][a];
       r = old + s_bcv[a][i] * F;
     }
   }
@@ -494,7 +616,7 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
 
   // ---- boundary sides: Dirichlet penalty (and Robin for T), one side at a time
   for (int sd = 0; sd < F::NSIDE; sd++) {
-    if (A.neigh[(long)e * F::NSIDE + sd] != -1) continue;
+    if (s_neigh[sd] != -1) continue;
     const int *sur = A.side.nodes[sd];
     const int last = sur[F::NSN - 1];
     const double det = jac_sur<DIM>(t, F::NSQ - 1, s_xx, sur);
@@ -529,17 +651,17 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
       if (s_bcv[a][last] == 0) {
         if (!ns) {
           const int bc_beta = s_bcb[0][last] % 2;
-          A.vv[blk] += ipen;
+          add_cg(A.vv + blk, ipen);
           if (mode == 1) A.rhs[nlv] += bc_beta * ipen * s_uold[0][lv];
         } else {
           const int bs = s_bcb[a][lv];
           const int bc_rhs = (bs & 4) >> 2, bc_tg = (bs & 2) >> 1, bc_n = bs % 2;
           double vdn = 0.;
           for (int d = 0; d < DIM; d++) vdn += nrm[d] * s_uold[d][lv];
-          A.vv[(long)(a * DIM + a) * A.nqq + blk] +=
-              ((1 - bc_n) * (1 - bc_tg) + bc_tg) * ipen + ipen * nrm[a] * nrm[a] * (bc_n - bc_tg);
+          add_cg(A.vv + (long)(a * DIM + a) * A.nqq + blk,
+                 ((1 - bc_n) * (1 - bc_tg) + bc_tg) * ipen + ipen * nrm[a] * nrm[a] * (bc_n - bc_tg));
           for (int b = a + 1; b < DIM; b++)
-            A.vv[(long)(a * DIM + b) * A.nqq + blk] += ipen * nrm[b] * nrm[a] * (bc_n - bc_tg);
+            add_cg(A.vv + (long)(a * DIM + b) * A.nqq + blk, ipen * nrm[b] * nrm[a] * (bc_n - bc_tg));
           if (mode == 1)
             A.rhs[(long)a * A.N + nlv] +=
                 bc_rhs * ipen *
@@ -568,7 +690,7 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
             diag += dt * bc_tg * phij * phii + dt * nrm[a] * nrm[a] * phij * phii * (bc_n - bc_tg);
           }
         }
-        A.vv[(long)(a * DIM + a) * A.nqq + blk] += diag;
+        add_cg(A.vv + (long)(a * DIM + a) * A.nqq + blk, diag);
         for (int b = a + 1; b < DIM; b++)  // normal-normal coupling, one column node at a time
           for (int j = 0; j < F::NSN; j++) {
             double o = 0.;
@@ -576,7 +698,7 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
               o += jac_sur<DIM>(t, q, s_xx, sur) * t->sw[q] * bcv2 * nrm[b] * nrm[a] * t->sphi[q][j] *
                    t->sphi[q][k] * (bc_n - bc_tg);
             const long bj = qq_ptr[nlv] + A.pos_qq[((long)e * NEN + lv) * NEN + sur[j]];
-            A.vv[(long)(a * DIM + b) * A.nqq + bj] += o;
+            add_cg(A.vv + (long)(a * DIM + b) * A.nqq + bj, o);
           }
         if (mode == 1 && ph.traction != 0.) A.rhs[(long)a * A.N + nlv] += fr;
       } else if (!ns && s_bcb[0][last] != 0) {
@@ -588,7 +710,7 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
           double v = 0.;
           for (int q = 0; q < F::NSQ; q++) v += jac_sur<DIM>(t, q, s_xx, sur) * t->sw[q] * t->sphi[q][k] * t->sphi[q][j];
           const long bj = qq_ptr[nlv] + A.pos_qq[((long)e * NEN + lv) * NEN + sur[j]];
-          A.vv[bj] += bv * bc_alpha * diff_t * v;
+          add_cg(A.vv + bj, bv * bc_alpha * diff_t * v);
         }
       }
     }
@@ -596,16 +718,17 @@ __device__ __forceinline__ void assemble_element(const AsmArgs<DIM> &A, const in
   }
 }
 
-template <int DIM, int NT>
-__global__ void __launch_bounds__(NT, DIM == 3 ? EXF_ASM_MINB3 : EXF_ASM_MINB2) k_assemble(AsmArgs<DIM> A, int mode) {
-  assemble_element<DIM, NT>(A, A.elist[blockIdx.x], mode);
+template <int DIM, int NT, bool NS>
+__global__ void __launch_bounds__(NT, asm_ctas<DIM>)
+    k_assemble(AsmArgs<DIM> A, int mode) {
+  assemble_element<DIM, NT, NS>(A, A.elist[blockIdx.x], mode);
 }
 
 // One colour of every level in one launch: work item {level, element}, the level's
 // arguments copied to shared memory (levels write separate matrices, so their elements of
 // one colour run together; each entry still receives its elements in colour order)
-template <int DIM, int NT>
-__global__ void __launch_bounds__(NT, DIM == 3 ? EXF_ASM_MINB3 : EXF_ASM_MINB2)
+template <int DIM, int NT, bool NS>
+__global__ void __launch_bounds__(NT, asm_ctas<DIM>)
     k_assemble_levels(const AsmArgs<DIM> *__restrict__ args, const int2 *__restrict__ work) {
   __shared__ AsmArgs<DIM> sA;
   static_assert(sizeof(AsmArgs<DIM>) % 4 == 0, "argument block copied in words");
@@ -614,7 +737,7 @@ __global__ void __launch_bounds__(NT, DIM == 3 ? EXF_ASM_MINB3 : EXF_ASM_MINB2)
   int *dst = reinterpret_cast<int *>(&sA);
   for (int k = threadIdx.x; k < (int)(sizeof(AsmArgs<DIM>) / 4); k += NT) dst[k] = src[k];
   __syncthreads();
-  assemble_element<DIM, NT>(sA, w.y, sA.rhs ? 1 : 0);
+  assemble_element<DIM, NT, NS>(sA, w.y, sA.rhs ? 1 : 0);
 }
 
 template <int DIM>
@@ -701,13 +824,14 @@ static int assemble_dim(exf_sys *s, const exf_phys *ph, int lev, int mode) {
   AsmArgs<DIM> a;
   EXF_TRY(level_args<DIM>(s, ph, lev, mode, a));
   const MeshLevel &ml = s->mesh->lev[lev];
-  constexpr int NT = DIM == 2 ? 128 : 256;
+  constexpr int NT = asm_threads;
   for (int c = 0; c + 1 < (int)ml.ecol_off.size(); c++) {
     int n = ml.ecol_off[c + 1] - ml.ecol_off[c];
     if (n == 0) continue;
     a.elist = ml.d_elist.p + ml.ecol_off[c];
     a.nel_c = n;
-    k_assemble<DIM, NT><<<n, NT, 0, s->stream>>>(a, mode);
+    if (s->kind == EXF_KIND_NS) k_assemble<DIM, NT, true><<<n, NT, 0, s->stream>>>(a, mode);
+    else k_assemble<DIM, NT, false><<<n, NT, 0, s->stream>>>(a, mode);
     EXF_LAUNCH_CHECK();
     EXF_COUNT(1);
   }
@@ -747,13 +871,15 @@ static int assemble_all_dim(exf_sys *s, const exf_phys *ph) {
   for (int l = 0; l < nl; l++) EXF_TRY(level_args<DIM>(s, ph, l, l == top ? 1 : 0, args[l]));
   EXF_TRY(s->asm_args.ensure(nl * sizeof(AsmArgs<DIM>)));
   EXF_CUDA(cudaMemcpyAsync(s->asm_args.p, args.data(), nl * sizeof(AsmArgs<DIM>), cudaMemcpyHostToDevice, s->stream));
-  constexpr int NT = DIM == 2 ? 128 : 256;
+  constexpr int NT = asm_threads;
   const AsmArgs<DIM> *d_args = reinterpret_cast<const AsmArgs<DIM> *>(s->asm_args.p);
   const int2 *d_work = reinterpret_cast<const int2 *>(s->asm_work.p);
   for (int c = 0; c + 1 < (int)s->asm_work_off.size(); c++) {
     const int n = s->asm_work_off[c + 1] - s->asm_work_off[c];
     if (n == 0) continue;
-    k_assemble_levels<DIM, NT><<<n, NT, 0, s->stream>>>(d_args, d_work + s->asm_work_off[c]);
+    const int2 *wk = d_work + s->asm_work_off[c];
+    if (s->kind == EXF_KIND_NS) k_assemble_levels<DIM, NT, true><<<n, NT, 0, s->stream>>>(d_args, wk);
+    else k_assemble_levels<DIM, NT, false><<<n, NT, 0, s->stream>>>(d_args, wk);
     EXF_LAUNCH_CHECK();
     EXF_COUNT(1);
   }
