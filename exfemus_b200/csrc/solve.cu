@@ -482,7 +482,8 @@ struct Packed16 {
 // up front with them.  rsc undoes a row scaling of the blocks on each lane's sum.
 // patch_row_first loads what does not change during a sweep (the couplings and the
 // first chunk), so a kernel can issue it before waiting for the iterate;
-// patch_row_rest gathers, multiplies and walks the remaining chunks.  LW >= RA and
+// patch_row_rest gathers, multiplies and walks the remaining chunks (VL > 1: lane l keeps
+// the sums of lanes l, l + LPR, ... of a VL LPR wide row apart).  LW >= RA and
 // VW >= RA * D are the caller's buffer widths.
 template <class T, int D, int LPR, int UNR, int RA, class BL, int LW, int VW>
 __device__ __forceinline__ void patch_row_first(int lane, int k0, int nk, int l0, int nl, const BL &bl,
@@ -504,12 +505,13 @@ __device__ __forceinline__ void patch_row_first(int lane, int k0, int nk, int l0
   }
 }
 
-template <class T, int D, int LPR, int UNR, bool I4, int RA, class BL, int LW, int VW>
+template <class T, int D, int LPR, int UNR, bool I4, int RA, int VL = 1, class BL, int LW, int VW>
 __device__ __forceinline__ void patch_row_rest(int lane, int N, int k0, int nk, int l0, int nl, const BL &bl,
                                                const int *__restrict__ ql_col, long lstride,
-                                               const T *__restrict__ lv, const T *__restrict__ x, T acc[D],
+                                               const T *__restrict__ lv, const T *__restrict__ x, T acc[VL * D],
                                                const T (&rsc)[D], int lc, const T (&lw)[LW], int (&c)[UNR],
                                                T (&v)[UNR][VW]) {
+  static_assert(UNR % VL == 0, "a chunk holds whole sets of lanes");
   for (int base = 0; base < nk; base += UNR * LPR) {
     if (base > 0) {
 #pragma unroll
@@ -539,22 +541,28 @@ __device__ __forceinline__ void patch_row_rest(int lane, int N, int k0, int nk, 
 #pragma unroll
         for (int a = 0; a < RA; a++)
 #pragma unroll
-          for (int bb = 0; bb < D; bb++) acc[a] += v[u][a * D + bb] * xb[u][bb];
+          for (int bb = 0; bb < D; bb++) acc[(u % VL) * D + a] += v[u][a * D + bb] * xb[u][bb];
   }
   if constexpr (BL::scaled) {
 #pragma unroll
-    for (int a = 0; a < RA; a++) acc[a] *= rsc[a];
+    for (int a = 0; a < RA; a++)
+#pragma unroll
+      for (int w = 0; w < VL; w++) acc[w * D + a] *= rsc[a];
   }
   if (lc >= 0) {
     const T pval = x[Lay<I4>::p(lc, N, D)];
 #pragma unroll
     for (int a = 0; a < RA; a++) acc[a] += lw[a] * pval;
   }
-  for (int i = LPR + lane; i < nl; i += LPR) {  // rows with more than LPR pressure couplings
-    const T pval = x[Lay<I4>::p(ql_col[l0 + i], N, D)];
+  for (int i0 = VL == 1 ? LPR : 0; i0 < nl; i0 += VL * LPR)  // rows with more than LPR pressure couplings
 #pragma unroll
-    for (int a = 0; a < RA; a++) acc[a] += lv[(long)a * lstride + l0 + i] * pval;
-  }
+    for (int w = 0; w < VL; w++) {
+      const int i = i0 + w * LPR + lane;
+      if (i < LPR || i >= nl) continue;
+      const T pval = x[Lay<I4>::p(ql_col[l0 + i], N, D)];
+#pragma unroll
+      for (int a = 0; a < RA; a++) acc[w * D + a] += lv[(long)a * lstride + l0 + i] * pval;
+    }
 }
 
 template <class T, int D, int LPR, int UNR, bool I4, int RA, class BL>
@@ -570,10 +578,11 @@ __device__ __forceinline__ void patch_row_dot(int lane, int N, int k0, int nk, i
 }
 
 // ROWS phase 1: residuals of the star rows (g < nrows) and of the patches' pressure
-// rows (g >= nrows), LPR lanes per row, written in patch order.  rinfo per star row:
+// rows (g >= nrows), LPR lanes per row, written in patch order; with VL = 2 a lane keeps
+// the sums of two lanes of a 2 LPR wide row, added in that row's order.  rinfo per star row:
 // {node, qq_ptr[node], ql_ptr[node], nqq | nql << 8 | tile index << 16}; pinfo per patch
 // (two int4): {m, first star entry, qq_ptr[m], ql_ptr[m]}, {nqq(m), nql(m), lattice, 0}.
-template <class T, int D, int LPR, int NT, bool I4, int UNR, int MINB, class VB>
+template <class T, int D, int LPR, int NT, bool I4, int UNR, int MINB, int VL, class VB>
 __global__ void __launch_bounds__(NT, MINB)
     k_vanka_rows(const int4 *__restrict__ rinfo, int nrows, int gbase, const int4 *__restrict__ pinfo, int npatch,
                  int N, VB vb, const T *__restrict__ vsc, const int *__restrict__ qq_col,
@@ -609,21 +618,27 @@ __global__ void __launch_bounds__(NT, MINB)
     patch_row_first<T, D, LPR, UNR, 1>(lane, q0.z, q1.x, q0.w, q1.y, pb, ql_col, 0, pp, lc, lw, c, v);
   }
   EXF_PDL_WAIT();
-  T acc[D], bv[D];
+  T acc[VL * D], bv[D];
 #pragma unroll
-  for (int a = 0; a < D; a++) acc[a] = bv[a] = T(0);
+  for (int a = 0; a < VL * D; a++) acc[a] = T(0);
+#pragma unroll
+  for (int a = 0; a < D; a++) bv[a] = T(0);
   if (vel) {
     if (lane == 0) {
 #pragma unroll
       for (int a = 0; a < D; a++) bv[a] = b[Lay<I4>::v(a, node, N)];
     }
-    patch_row_rest<T, D, LPR, UNR, I4, D>(lane, N, q0.y, q0.w & 0xff, q0.z, (q0.w >> 8) & 0xff, vb, ql_col, nql, vp,
+    patch_row_rest<T, D, LPR, UNR, I4, D, VL>(lane, N, q0.y, q0.w & 0xff, q0.z, (q0.w >> 8) & 0xff, vb, ql_col, nql, vp,
                                           x, acc, sc, lc, lw, c, v);
   } else if (prs) {
     if (lane == 0) bv[0] = b[Lay<I4>::p(node, N, D)];
     const T one[D] = {};
-    patch_row_rest<T, D, LPR, UNR, I4, 1>(lane, N, q0.z, q1.x, q0.w, q1.y, pb, ql_col, 0, pp, x, acc, one, lc, lw, c,
+    patch_row_rest<T, D, LPR, UNR, I4, 1, VL>(lane, N, q0.z, q1.x, q0.w, q1.y, pb, ql_col, 0, pp, x, acc, one, lc, lw, c,
                                           v);
+  }
+  if constexpr (VL == 2) {
+#pragma unroll
+    for (int a = 0; a < D; a++) acc[a] += acc[D + a];
   }
 #pragma unroll
   for (int a = 0; a < D; a++)
@@ -1789,12 +1804,18 @@ static int vanka_sweep_rows(exf_sys *s, int lev, const exf_mg_params *p, T *x, c
   constexpr int SU = D == 3 ? (375 + NTS - 1) / NTS : 1;  // 3D stars: 125 nodes x 3; 2D: 25 x 2 <= 64
   constexpr int LPR = D == 3 ? 32 : 16;
   constexpr int NTR = 256;
-  constexpr int UNR_S = sizeof(T) == 4 ? EXF_UNR_BIG32 : EXF_UNR_BIG64;
+  constexpr bool ROWS64 = D == 2 && sizeof(T) == 8;
+  constexpr int UNR_S = ROWS64 ? 2 : sizeof(T) == 4 ? EXF_UNR_BIG32 : EXF_UNR_BIG64;
 #ifndef EXF_LPR_BIG32
 #define EXF_LPR_BIG32 16
 #endif
   constexpr int LPR_S = (D == 3 && sizeof(T) == 4) ? EXF_LPR_BIG32 : LPR;
-  constexpr int MINB_S = sizeof(T) == 4 ? EXF_MINB_BIG32 : EXF_MINB_BIG64;
+  // FP64 levels above one wave of rows in 2D: 8 lanes hold the sums of 16 (bits unchanged),
+  // so a row's 25 blocks of 4 doubles are two rounds of two loads in half as many threads:
+  // 257 x 257 sweep 159 -> 133 us (CTAs per SM 4; 5: 139, 6: 148).  FP32 gains nothing
+  // (98 -> 101 us, 513 x 513 336 -> 339 us) and keeps 16 lanes.
+  constexpr int VL_S = ROWS64 ? 2 : 1;
+  constexpr int MINB_S = ROWS64 ? 4 : sizeof(T) == 4 ? EXF_MINB_BIG32 : EXF_MINB_BIG64;
   // 3D FP32 levels of one to four waves: two blocks per lane, 64 registers
 #ifndef EXF_UNR_MID32
 #define EXF_UNR_MID32 2
@@ -1920,11 +1941,11 @@ static int vanka_sweep_rows(exf_sys *s, int lev, const exf_mg_params *p, T *x, c
       if (!p->fp32_blocks) {
         using VB = Packed16<D>;
         const VB vb{L.qq_col.p, L.h16.p, L.h16cx.p};
-        auto kern = big   ? k_vanka_rows<T, D, LPR_S, NTR, I4, UNR_S, MINB_S, VB>
-                    : mid ? k_vanka_rows<T, D, LPR_M, NTR, I4, UNR_M, MINB_M, VB>
-                          : k_vanka_rows<T, D, LPR_L, NTR, I4, UNR_L, 1, VB>;
+        auto kern = big   ? k_vanka_rows<T, D, LPR_S / VL_S, NTR, I4, UNR_S, MINB_S, VL_S, VB>
+                    : mid ? k_vanka_rows<T, D, LPR_M, NTR, I4, UNR_M, MINB_M, 1, VB>
+                          : k_vanka_rows<T, D, LPR_L, NTR, I4, UNR_L, 1, 1, VB>;
         const long nthr_k = big ? nthr_s : (long)(nr + n) * (mid ? LPR_M : LPR_L);
-        EXF_CUDA(launch_pdl(kern, dim3(nblk(nthr_k, NTR)), dim3(NTR), 0, s->stream,
+        EXF_CUDA(launch_pdl(kern, dim3(nblk(big ? nthr_k / VL_S : nthr_k, NTR)), dim3(NTR), 0, s->stream,
                             L.vrinfo.p + L.vrow_off[c], nr, L.vrow_off[c], pin, n, L.N, vb, (const T *)L.vsc.p,
                             L.qq_col.p, L.ql_col.p, L.nql, L.nqqL, VT<T>::vp(L), VT<T>::pv(L), VT<T>::pp(L), x, b,
                             res, pres_off));
@@ -1934,9 +1955,9 @@ static int vanka_sweep_rows(exf_sys *s, int lev, const exf_mg_params *p, T *x, c
     if (!launched) {  // FP64, or FP32 storage of the blocks in the FP32 V-cycle
       using VB = PlanarBlocks<T, D * D>;
       const VB vb{L.qq_col.p, VT<T>::vv(L), L.nqq};
-      auto kern = big ? k_vanka_rows<T, D, LPR, NTR, I4, UNR_S, MINB_S, VB>
-                      : k_vanka_rows<T, D, LPR, NTR, I4, UNR_L, 1, VB>;
-      EXF_CUDA(launch_pdl(kern, dim3(nblk(nthr, NTR)), dim3(NTR), 0, s->stream, L.vrinfo.p + L.vrow_off[c], nr,
+      auto kern = big ? k_vanka_rows<T, D, LPR / VL_S, NTR, I4, UNR_S, MINB_S, VL_S, VB>
+                      : k_vanka_rows<T, D, LPR, NTR, I4, UNR_L, 1, 1, VB>;
+      EXF_CUDA(launch_pdl(kern, dim3(nblk(big ? nthr / VL_S : nthr, NTR)), dim3(NTR), 0, s->stream, L.vrinfo.p + L.vrow_off[c], nr,
                           L.vrow_off[c], pin, n, L.N, vb, (const T *)nullptr, L.qq_col.p, L.ql_col.p, L.nql, L.nqqL,
                           VT<T>::vp(L), VT<T>::pv(L), VT<T>::pp(L), x, b, res, pres_off));
     }
