@@ -353,6 +353,8 @@ struct exf_sys {
   // exf_assemble_all: per colour the {level, element} work list of every level (top level
   // first) and the levels' argument blocks
   exf::DBuf<unsigned char> asm_work, asm_args;
+  exf::DBuf<double> resid_vec;  // exf_resid's x, b and r
+  std::mutex resid_mu;          // held while a call uses them
   std::vector<int> asm_work_off;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t user_ev[8] = {nullptr};
