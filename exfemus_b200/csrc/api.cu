@@ -82,15 +82,21 @@ static int nb_csr(exf_sys *s, int lev, double *d_vals, int dir) {
 int csr_values(exf_sys *s, int lev, double *d_out) { return nb_csr(s, lev, d_out, 0); }
 int csr_set_values(exf_sys *s, int lev, const double *d_in) { return nb_csr(s, lev, const_cast<double *>(d_in), 1); }
 
-__global__ void k_d2f(const double *a, float *b, long n) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = (float)a[i];
+// FP32 copy, four entries a thread in 16-byte words (both arrays are whole allocations)
+__global__ void k_d2f(const double *__restrict__ a, float *__restrict__ b, long n) {
+  const long i = 4 * ((long)blockIdx.x * blockDim.x + threadIdx.x);
+  if (i + 4 <= n) {
+    const double2 u = *reinterpret_cast<const double2 *>(a + i), w = *reinterpret_cast<const double2 *>(a + i + 2);
+    *reinterpret_cast<float4 *>(b + i) = make_float4((float)u.x, (float)u.y, (float)w.x, (float)w.y);
+  } else {
+    for (long k = i; k < n; k++) b[k] = (float)a[k];
+  }
 }
 int sync_fp32(exf_sys *s, int lev) {
   SysLevel &L = s->L[lev];
   auto cp = [&](const DBuf<double> &a, DBuf<float> &b) {
     if (a.p && b.p) {
-      k_d2f<<<nblk(a.n, 256), 256, 0, s->stream>>>(a.p, b.p, a.n);
+      k_d2f<<<nblk((a.n + 3) / 4, 256), 256, 0, s->stream>>>(a.p, b.p, a.n);
       EXF_COUNT(1);
     }
   };
