@@ -180,15 +180,16 @@ struct Transfer {
   std::vector<double> h_val;
 };
 
-// A scalar level as the cluster kernel reads it (mg_cluster.cu): positions are the nodes in
-// colour order, padded to whole warps; a step deals one round of a colour's rows to the row
-// groups of `act` CTAs
+// A scalar level as the cluster kernel reads it (mg_cluster.cu, mg_cluster_plan.h): positions
+// are the nodes in colour order, padded to whole warps; a step deals one round of a colour's
+// rows to the row groups of `act` CTAs
 struct CluTable {
   bool ok = false;
-  int act = 1, steps = 0, Np = 0, entries = 0;  // CTAs, steps of a sweep, positions, most entries of a
-                                                // CTA (0: too many for its shared memory)
+  int act = 1, steps = 0, exch = 0, Np = 0, entries = 0;  // CTAs, steps and exchanges of a sweep, positions,
+                                                          // most entries of a CTA (0: too many for its
+                                                          // shared memory)
   DBuf<int4> mem;    // the tables below, behind one another
-  const int4 *tab = nullptr;   // [act][steps][groups] {position or -1, first entry, entries, diagonal - first}
+  const int4 *tab = nullptr;   // [act][steps][groups] {position or -1, first entry, entries (0: padding), diagonal - first}
   const int *first = nullptr;  // [act][steps][groups] first of the row's entries in the CTA's copy
   const int2 *ent = nullptr;   // [act][entries] the copy's entries: {entry of the matrix, position of its column}
   const int2 *step = nullptr;  // {positions of the colour, 1: last step of it, 2: first step of it}

@@ -26,6 +26,7 @@
 
 #include "cluster.cuh"
 #include "exf_internal.h"
+#include "mg_cluster_plan.h"
 
 namespace exf {
 
@@ -40,13 +41,13 @@ static constexpr int clu_lpr(int dim) { return dim == 2 ? 8 : 16; }
 
 template <class T>
 struct CluLevel {
-  int N, Np, steps, act, mat;  // nodes, padded positions, steps of a sweep, active CTAs, entries
-                               // of a CTA's rows in shared memory (0: not there)
+  int N, Np, steps, exch, act, mat;  // nodes, padded positions, steps and exchanges of a sweep, active
+                                     // CTAs, entries of a CTA's rows in shared memory (0: not there)
   const int4 *tab;             // CluTable
   const int *first;
   const int2 *ent;
   const int2 *step;
-  const int *node;
+  const int *node;             // -1: padding
   const int *col;              // positions of the columns
   const T *vv;
   T *x, *b, *r;
@@ -82,8 +83,8 @@ __device__ __forceinline__ void phase_sync(int act) {
 
 // A level as a CTA holds it in shared memory: the iterate by position (colour order), and
 // step after step the row of each of the CTA's groups: {position or -1, first entry,
-// entries, diagonal entry - first entry}, the reciprocal of the diagonal entry and the rhs;
-// where they fit (mat), the rows' entries too.
+// entries (0: padding), diagonal entry - first entry}, the reciprocal of the diagonal entry
+// and the rhs; where they fit (mat), the rows' entries too.
 template <class T>
 struct CluSmem {
   T *x;
@@ -142,7 +143,7 @@ __device__ __forceinline__ void load_level(const CluLevel<T> &L, int rank, CluSm
   for (int q = threadIdx.x; q < n; q += kCluNT) {
     const int4 d = tab[q];
     T inv = T(0), b = T(0);
-    if (d.x >= 0) {
+    if (d.z > 0) {
       inv = T(1) / L.vv[d.y + d.w];
       b = L.b[L.node[d.x]];
     }
@@ -175,12 +176,19 @@ __device__ __forceinline__ void store_x(const CluLevel<T> &L, int gt, int nth, c
 }
 
 // nsw sweeps of one level: the steps of all sweeps form one sequence.  With several CTAs a
-// warp's new values are sent to every CTA; a CTA starts a colour when all values of the
-// previous one have arrived.  No CTA can then overwrite a value that another still reads:
-// it has that CTA's values of the colour, which were sent after its reads.  Two mbarriers
-// alternate, since a value of the next colour may arrive before the last of the current
-// one (of the colour after that, it cannot).  Entries that are not in shared memory (!MAT)
-// are loaded two or three steps ahead.
+// warp's new values are sent to every CTA, and a warp starts a colour when the CTA's mbarrier
+// of the colour before has completed.  Colours alternate between two mbarriers; a phase p
+// completes when all of colour p's bytes have arrived AND each of the CTA's warps has
+// arrived, which a warp does after it has seen phase p - 2.  Two rules keep the order:
+//  * no warp is left behind: phase p + 2 waits for the arrival of every warp of the CTA, so
+//    its parity cannot turn back under a warp that still tests phase p (a warp without rows
+//    in two colours running would otherwise wait for a phase that is over);
+//  * no value arrives early: a CTA sends colour p + 2 after its phase p + 1, hence after the
+//    sends of colour p + 1 of EVERY CTA (plan_cluster deals each CTA a unit in each colour,
+//    padding if need be), hence after phase p of every CTA: its bytes cannot count as colour
+//    p's, nor can it overwrite a value that a warp still reads for colour p + 1 (that warp
+//    has not sent yet).
+// Entries that are not in shared memory (!MAT) are loaded two or three steps ahead.
 template <class T, int LPR, int E, bool MAT>
 __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int reverse, CluSmem<T> &S) {
   constexpr int GC = kCluNT / LPR, RW = 32 / LPR;
@@ -195,18 +203,23 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
   const T *sinv = S.inv + g, *sb = S.b + g;
   // step i of a sweep is step s0 + i * dir of the tables
   const int s0 = reverse ? steps - 1 : 0, dir = reverse ? -1 : 1;
-  // thread 0 arms the mbarriers two colours ahead of the exchange
-  int ai = 0;  // next step to look at, of all sweeps
+  // the warps arrive for a colour once they have sent the colour before (while its values
+  // travel), thread 0 with the colour's bytes
+  int ai = 0, left = nsw * L.exch;  // next step to look at, of all sweeps; colours to arrive for
   unsigned aph = S.phase;
   auto arm = [&]() {
-    while (ai < total) {
-      const int2 st = S.step[s0 + (ai % steps) * dir];
-      ai++;
-      if (st.y & bit) {
-        mbar_arrive_tx(&S.bar[aph++ & 1], (unsigned)(st.x * sizeof(T)));
-        return;
-      }
+    if (wl > 0 || left <= 0 || !S.ok) return;
+    if (threadIdx.x > 0) {
+      mbar_arrive(&S.bar[aph & 1]);
+    } else {
+      int2 st;
+      do {
+        st = S.step[s0 + (ai++ % steps) * dir];
+      } while (!(st.y & bit));
+      mbar_arrive_tx(&S.bar[aph & 1], (unsigned)(st.x * sizeof(T)));
     }
+    aph++;
+    left--;
   };
   const unsigned dst = (unsigned)wl / PK;  // the CTA this lane sends to, its vector
   const int hv = wl % PK;
@@ -216,10 +229,7 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
     ax = cluster_addr(S.x + hv * VL, dst);
     ab = cluster_addr(S.bar, dst);
   }
-  if (L.act > 1 && threadIdx.x == 0) {
-    arm();
-    arm();
-  }
+  if (L.act > 1) arm();
   RowSlot<T, E> s[PF];
   int ld = s0, nld = 0;  // table step of the next load
   auto load = [&](RowSlot<T, E> &r) {
@@ -250,10 +260,10 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
             const T v0 = __shfl_sync(0xffffffffu, xn, (hv * VL) * LPR);
             const T v1 = __shfl_sync(0xffffffffu, xn, (hv * VL + 1) * LPR);
             if constexpr (VL == 2) {
-              if (sender) cluster_send2(at, v0, v1, bar);
+              if (sender && S.ok) cluster_send2(at, v0, v1, bar);
             } else {
               const T v2 = __shfl_sync(0xffffffffu, xn, 2 * LPR), v3 = __shfl_sync(0xffffffffu, xn, 3 * LPR);
-              if (sender) cluster_send4(at, v0, v1, v2, v3, bar);
+              if (sender && S.ok) cluster_send4(at, v0, v1, v2, v3, bar);
             }
           }
         }
@@ -267,12 +277,12 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
           if (L.act == 1) {
             __syncthreads();
           } else {
+            arm();
             if (S.ok && !mbar_wait(&S.bar[S.phase & 1], (S.phase >> 1) & 1)) {
-              S.ok = false;  // leave by the regular path, without further waits
+              S.ok = false;  // leave by the regular path, without further waits, sends or arrivals
               atomicExch(S.wait_flag, 1);
             }
             S.phase++;
-            if (threadIdx.x == 0) arm();
           }
         }
       }
@@ -308,8 +318,8 @@ __global__ void __launch_bounds__(kCluNT, 1) k_mg_cluster(const __grid_constant_
   S.wait_flag = A.wait_flag;
   S.ok = true;
   if (tid == 0) {
-    mbar_init(&s_bar[0], 1);
-    mbar_init(&s_bar[1], 1);
+    mbar_init(&s_bar[0], kCluNT / 32);
+    mbar_init(&s_bar[1], kCluNT / 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (csize > 1) {  // every CTA's mbarriers exist before the first value is sent
@@ -342,7 +352,7 @@ __global__ void __launch_bounds__(kCluNT, 1) k_mg_cluster(const __grid_constant_
         RowSlot<T, E> s;
         load_row<T, LPR, E, true>(col, vv, q, lane, s);
         const T acc = row_dot<T, LPR, E, true>(col, vv, s, q, lane, S.x);
-        if (q.x >= 0 && lane == 0) L.r[L.node[q.x]] = S.b[at] - acc;
+        if (q.z > 0 && lane == 0) L.r[L.node[q.x]] = S.b[at] - acc;
       }
       store_x(L, gt, nth, S);
     }
@@ -481,9 +491,7 @@ __global__ void k_clu_entries(const int4 *tab, const int *first, int ntab, int p
   for (int i = threadIdx.x % 8; i < d.z; i += 8) o[i] = make_int2(d.y + i, col[d.y + i]);
 }
 
-// Tables of a scalar level for the cluster kernel, once per system: positions (a colour's
-// rows longest first, so that a warp's rows are alike, each colour padded to whole warps)
-// and the rows of each CTA's groups, a colour's warps dealt round-robin to the CTAs.
+// Tables of a scalar level for the cluster kernel, once per system (plan_cluster)
 int build_cluster(exf_sys *s, int lev, const std::vector<int> &items) {
   SysLevel &L = s->L[lev];
   CluTable &C = L.clu;
@@ -502,51 +510,14 @@ int build_cluster(exf_sys *s, int lev, const std::vector<int> &items) {
   EXF_CUDA(cudaMemcpyAsync(qp.data(), L.qq_ptr.p, qp.size() * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   EXF_CUDA(cudaMemcpyAsync(diag.data(), L.diag_pos.p, diag.size() * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   EXF_CUDA(cudaStreamSynchronize(s->stream));
-  const int lpr = clu_lpr(s->dim), gc = kCluNT / lpr, rw = 32 / lpr, nw = kCluNT / 32;
-  int rows = 0;
-  for (int c = 0; c < L.ncolour; c++) rows = std::max(rows, L.col_off[c + 1] - L.col_off[c]);
-  // CTA 0 alone where a colour's rows fit its groups (its barrier costs a fifth of an
-  // exchange), otherwise the whole cluster (just enough CTAs for the rows: 2-6% slower)
-  C.act = rows <= gc ? 1 : most;
-  std::vector<int> node, pos(L.N, -1);
-  std::vector<int2> step;
-  std::vector<int> cbase(L.ncolour), rounds(L.ncolour);
-  for (int c = 0; c < L.ncolour; c++) {
-    const int n = L.col_off[c + 1] - L.col_off[c], units = (n + rw - 1) / rw;
-    std::vector<int> r(items.begin() + L.col_off[c], items.begin() + L.col_off[c + 1]);
-    std::stable_sort(r.begin(), r.end(), [&](int a, int b) { return qp[a + 1] - qp[a] > qp[b + 1] - qp[b]; });
-    cbase[c] = (int)node.size();
-    for (int k = 0; k < units * rw; k++) {
-      if (k < n) pos[r[k]] = (int)node.size();
-      node.push_back(k < n ? r[k] : -1);
-    }
-    rounds[c] = (units + C.act * nw - 1) / (C.act * nw);
-    for (int k = 0; k < rounds[c]; k++)
-      step.push_back(make_int2(units * rw, (k == rounds[c] - 1 ? 1 : 0) | (k == 0 ? 2 : 0)));
-  }
-  C.Np = (int)node.size();
-  C.steps = (int)step.size();
-  std::vector<int4> tab((size_t)C.act * C.steps * gc, make_int4(-1, 0, 0, -1));
-  int st0 = 0;
-  for (int c = 0; c < L.ncolour; c++) {
-    const int n = L.col_off[c + 1] - L.col_off[c];
-    for (int k = 0; k < n; k++) {
-      const int u = k / rw, cta = u % C.act, w = (u / C.act) % nw, rnd = u / C.act / nw;
-      const int v = node[cbase[c] + k];
-      tab[((size_t)cta * C.steps + st0 + rnd) * gc + w * rw + k % rw] =
-          make_int4(cbase[c] + k, qp[v], qp[v + 1] - qp[v], diag[v] - qp[v]);
-    }
-    st0 += rounds[c];
-  }
-  std::vector<int> first(tab.size(), 0);
-  for (int r = 0; r < C.act; r++) {
-    int at = 0;
-    for (size_t q = (size_t)r * C.steps * gc; q < (size_t)(r + 1) * C.steps * gc; q++) {
-      first[q] = at;
-      at += tab[q].z;
-    }
-    C.entries = std::max(C.entries, (at + 3) & ~3);
-  }
+  const int lpr = clu_lpr(s->dim), gc = kCluNT / lpr;
+  const CluPlan P = plan_cluster(L.N, qp.data(), diag.data(), L.ncolour, L.col_off.data(), items.data(), lpr, kCluNT,
+                                 most);
+  C.act = P.act;
+  C.Np = (int)P.node.size();
+  C.steps = (int)P.step.size();
+  C.exch = P.exch;
+  C.entries = P.entries;
   // entries that fit no CTA's shared memory are read from the level's arrays
   if ((size_t)C.entries * (4 + sizeof(float)) > kCluSmem) C.entries = 0;
   // one block of device memory, each table 16-byte aligned: tab, first, step, node, the
@@ -558,7 +529,9 @@ int build_cluster(exf_sys *s, int lev, const std::vector<int> &items) {
     if (bytes) memcpy(&mem[at], h.data(), bytes);
     return at;
   };
-  const size_t o_tab = put(tab), o_first = put(first), o_step = put(step), o_node = put(node), o_pos = put(pos);
+  static_assert(sizeof(CluRow) == sizeof(int4) && sizeof(CluStep) == sizeof(int2), "tables are copied as they are");
+  const size_t o_tab = put(P.tab), o_first = put(P.first), o_step = put(P.step), o_node = put(P.node),
+               o_pos = put(P.pos);
   const size_t o_col = mem.size(), o_ent = o_col + ((size_t)L.nqq + 3) / 4;
   EXF_TRY(C.mem.alloc(o_ent + (size_t)C.act * C.entries / 2));
   EXF_CUDA(cudaMemcpyAsync(C.mem.p, mem.data(), mem.size() * sizeof(int4), cudaMemcpyHostToDevice, s->stream));
@@ -619,6 +592,7 @@ int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi, bool zero
     if (l == 0) break;
     d.Np = L.clu.Np;
     d.steps = L.clu.steps;
+    d.exch = L.clu.exch;
     d.act = L.clu.act;
     d.tab = L.clu.tab;
     d.first = L.clu.first;

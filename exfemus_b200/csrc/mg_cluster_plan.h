@@ -1,0 +1,87 @@
+// mg_cluster_plan.h -- which CTA, warp and step of the cluster kernel (mg_cluster.cu) updates
+// which row of a scalar level.  Host code on plain arrays, no CUDA types, so that the rules
+// the kernel's exchange rests on can be checked without a device.
+#pragma once
+#include <algorithm>
+#include <cstdint>
+#include <vector>
+
+namespace exf {
+
+struct CluRow {  // a row group's row in one step
+  int pos, k0, len, diag;  // position or -1 (none), first entry, entries (0: padding), diagonal - first
+};
+struct CluStep {
+  int count, flags;  // positions of the colour; 1: last step of it, 2: first step of it
+};
+struct CluPlan {
+  int act = 1;      // CTAs that share the level
+  int exch = 0;     // colours with rows: exchanges of a sweep
+  int entries = 0;  // most matrix entries of a CTA, a multiple of 4
+  std::vector<int> node, pos;  // node at each position (-1 padding), position of each node
+  std::vector<CluStep> step;   // steps of a sweep
+  std::vector<CluRow> tab;     // [act][steps][groups]
+  std::vector<int> first;      // [act][steps][groups] first of the row's entries in the CTA's copy
+};
+
+// qp: row pointers, diag: absolute diagonal entries, items: the nodes by colour; lpr lanes
+// per row, CTAs of nt threads, `most` CTAs in the cluster.
+//
+// Positions are the nodes in colour order (a colour's rows longest first, so that a warp's
+// rows are alike, each colour padded to whole warps); a colour's units of one warp are dealt
+// round-robin to the CTAs.  A CTA's send in a colour tells the others that it has seen the
+// colour before complete, and its two mbarriers serve alternate colours: so EVERY CTA has a
+// unit in EVERY colour.  A colour with fewer units than CTAs gets units of padding.
+inline CluPlan plan_cluster(int N, const int *qp, const int *diag, int ncolour, const int *col_off, const int *items,
+                            int lpr, int nt, int most) {
+  CluPlan P;
+  const int gc = nt / lpr, rw = 32 / lpr, nw = nt / 32;
+  int rows = 0;
+  for (int c = 0; c < ncolour; c++) rows = std::max(rows, col_off[c + 1] - col_off[c]);
+  // CTA 0 alone where a colour's rows fit its groups (its barrier costs a fifth of an
+  // exchange), otherwise the whole cluster (just enough CTAs for the rows: 2-6% slower)
+  P.act = rows <= gc ? 1 : most;
+  P.pos.assign(N, -1);
+  std::vector<int> cbase(ncolour), rounds(ncolour), units(ncolour);
+  for (int c = 0; c < ncolour; c++) {
+    const int n = col_off[c + 1] - col_off[c];
+    units[c] = (n + rw - 1) / rw;
+    if (n > 0 && P.act > 1) units[c] = std::max(units[c], P.act);
+    std::vector<int> r(items + col_off[c], items + col_off[c + 1]);
+    std::stable_sort(r.begin(), r.end(), [&](int a, int b) { return qp[a + 1] - qp[a] > qp[b + 1] - qp[b]; });
+    cbase[c] = (int)P.node.size();
+    for (int k = 0; k < units[c] * rw; k++) {
+      if (k < n) P.pos[r[k]] = (int)P.node.size();
+      P.node.push_back(k < n ? r[k] : -1);
+    }
+    rounds[c] = (units[c] + P.act * nw - 1) / (P.act * nw);
+    for (int k = 0; k < rounds[c]; k++)
+      P.step.push_back({units[c] * rw, (k == rounds[c] - 1 ? 1 : 0) | (k == 0 ? 2 : 0)});
+    P.exch += n > 0;
+  }
+  const int steps = (int)P.step.size();
+  P.tab.assign((size_t)P.act * steps * gc, CluRow{-1, 0, 0, -1});
+  int st0 = 0;
+  for (int c = 0; c < ncolour; c++) {
+    for (int k = 0; k < units[c] * rw; k++) {
+      const int u = k / rw, cta = u % P.act, w = (u / P.act) % nw, rnd = u / P.act / nw;
+      const int p = cbase[c] + k, v = P.node[p];
+      CluRow &t = P.tab[((size_t)cta * steps + st0 + rnd) * gc + w * rw + k % rw];
+      if (v >= 0) t = {p, qp[v], qp[v + 1] - qp[v], diag[v] - qp[v]};
+      else if (k % rw == 0) t = {p, 0, 0, -1};  // a unit of padding: it sends, nothing reads it
+    }
+    st0 += rounds[c];
+  }
+  P.first.assign(P.tab.size(), 0);
+  for (int r = 0; r < P.act; r++) {
+    int at = 0;
+    for (size_t q = (size_t)r * steps * gc; q < (size_t)(r + 1) * steps * gc; q++) {
+      P.first[q] = at;
+      at += P.tab[q].len;
+    }
+    P.entries = std::max(P.entries, (at + 3) & ~3);
+  }
+  return P;
+}
+
+}  // namespace exf
