@@ -272,6 +272,7 @@ struct SysLevel {
   DBuf<uint4> ilu_str;
   DBuf<int2> ilu_src, ilu_chunk;
   int ilu_nsrc = 0, ilu_nchunk = 0, ilu_nrec[2] = {0, 0};
+  uint4 ilu_first = {0u, 0u, 0u, 0u};  // places of the first records
   // levels whose rows have at most kFacMax entries up to the diagonal: the rows of the
   // dense blocks of the factorisation, {entry, place} (k_ilu_struct), and the level offsets
   DBuf<int2> ilu_ent;

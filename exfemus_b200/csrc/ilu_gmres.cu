@@ -38,6 +38,7 @@
 
 #include "cluster.cuh"
 #include "exf_internal.h"
+#include "ilu_stream.h"
 
 namespace exf {
 
@@ -420,24 +421,26 @@ __global__ void __launch_bounds__(128) k_ilu_upper(int N, const int *__restrict_
 // L2 between warps (the kernels above).  Here a few warps solve in turn, a thread per row,
 // doing the reference's operations in the reference's order, and the values stay in shared
 // memory.  Their instructions are then the bound, so the factor comes as a stream in the order of its
-// use (another warp copies it into shared-memory stages): records of up to 32 rows of one
-// level and up to kTriE entries of each, in planes of 32 (constant strides):
-//   {groups of 4 entries, 1: first of its rows | 2: last | 4: last of its chunk, 16-byte
-//   words, 0}, row[32],
-//   1 / d [32], d[32], index[entries][32], value[entries][32]
-// A row of more entries continues in the next record.  Absent entries and rows point to a
-// zero behind the vector (s - 0 * 0 leaves the bits of s).  v holds c, then
-// w = (D + L)^-1 c, then y, in place: a row reads its own c (w) before it replaces it.
-constexpr int kTriE = 24, kTriStages = 4, kTriThreads = 256, kTriWarps = 4;
-constexpr int tri_words(int M) { return 41 + 24 * M; }  // M: a multiple of 4
-constexpr int kTriWords = 2 * tri_words(kTriE);  // a stage: two records at least
+// use (another warp copies it into shared-memory stages), in records of up to 32 rows of one
+// level (build_tri_stream).  Absent entries and rows point to a zero behind the vector
+// (s - 0 * 0 leaves the bits of s).  v holds c, then w = (D + L)^-1 c, then y, in place: a
+// row reads its own c (w) before it replaces it.
+//
+// The owner of a chunk's last record frees the chunk's stage.  By then every record of the
+// chunk has been solved, hence loaded, and no warp has anything else to read there: a record
+// holds the place of its warp's next one.  A warp's test of a stage's phase is safe too: the
+// chunk it waits for holds its own unsolved record, so the stage cannot have moved on, and
+// the chunk before it in the stage is not later than that of the record it has just solved
+// (kTriStages = kTriWarps), so that one was there.
+constexpr int kTriThreads = 256;
+static_assert(kTriStages >= kTriWarps, "a warp's next record is at most kTriWarps chunks on");
+static_assert(sizeof(TriWord) == sizeof(uint4) && sizeof(TriPair) == sizeof(int2), "streams are copied as they are");
 constexpr size_t kTriSmem = 224 * 1024;
 
 struct TriSmem {
   uint4 st[kTriStages][kTriWords];
   uint64_t full[kTriStages], empty[kTriStages], turn[kTriWarps];
-  double part[32];        // sums of rows that continue in the next record
-  int words[kTriStages];  // of the chunk in each stage
+  double part[32];  // sums of rows that continue in the next record
 };
 struct TriRow {  // a lane's row of a record, loaded a record ahead
   int g, flags, i;
@@ -491,7 +494,8 @@ __device__ __forceinline__ void tri_solve(const TriRow &t, double *v, double *pa
 
 __global__ void __launch_bounds__(kTriThreads) k_ilu_tri(int N, const uint4 *__restrict__ str,
                                                          const int2 *__restrict__ chunk, int nch, int nlo, int nrec,
-                                                         const double *c, double *y, int *err, const int *skip) {
+                                                         const uint4 first, const double *c, double *y, int *err,
+                                                         const int *skip) {
   if (skip && *skip) return;
   extern __shared__ __align__(16) unsigned char tri_raw[];
   TriSmem &S = *reinterpret_cast<TriSmem *>(tri_raw);
@@ -519,7 +523,6 @@ __global__ void __launch_bounds__(kTriThreads) k_ilu_tri(int N, const uint4 *__r
         ok = false;
         break;
       }
-      S.words[k] = ch.y;
       mbar_arrive_tx(&S.full[k], (unsigned)ch.y * 16u);
       bulk_g2s(&S.st[k][0], str + ch.x, (unsigned)ch.y * 16u, &S.full[k]);
       if (it + 1 < nch) ch = chunk[it + 1];
@@ -530,37 +533,26 @@ __global__ void __launch_bounds__(kTriThreads) k_ilu_tri(int N, const uint4 *__r
     }
   } else if (warp < kTriWarps) {
     // the warps solve the records in turn; while one solves, the others load their next
-    int it = -1, o = 0, words = 0;  // the newest chunk looked at, the place of its next record
-    bool good = true;
-    auto next_record = [&](uint4 &h) -> const uint4 * {  // nullptr after a wait that ran out
-      if (o >= words && good) {
-        it++;
-        const int k = it % kTriStages;
-        if (!mbar_wait(&S.full[k], (it / kTriStages) & 1)) {
-          atomicExch(err, 1);
-          good = false;
-        }
-        o = 0;
-        words = S.words[k];
-      }
-      if (!good) return nullptr;
-      const uint4 *r = &S.st[it % kTriStages][o];
-      h = r[0];
-      o += (int)h.z;
-      return r;
-    };
     TriRow t;
     int ci = 0;  // chunk of the record in hand
-    bool have = false;
-    auto fetch = [&](int skip) {
-      uint4 h;
-      for (int q = 0; q < skip; q++) next_record(h);
-      const uint4 *r = next_record(h);
-      have = r != nullptr;
-      ci = it;
-      if (have) tri_load(t, r, h, lane);
+    bool good = true, have = false;
+    static_assert(kTriWarps == 4, "a first place for each warp");
+    unsigned next = warp == 0 ? first.x : warp == 1 ? first.y : warp == 2 ? first.z : first.w;
+    auto fetch = [&]() {
+      ci += next >> 24;
+      const int k = ci % kTriStages;
+      if (good && !mbar_wait(&S.full[k], (ci / kTriStages) & 1)) {
+        atomicExch(err, 1);
+        good = false;
+      }
+      have = good;
+      if (!have) return;
+      const uint4 *r = &S.st[k][next & 0xffffffu];
+      const uint4 h = r[0];
+      next = h.w;
+      tri_load(t, r, h, lane);
     };
-    if (warp < nrec) fetch(warp);
+    if (warp < nrec) fetch();
     for (int k = warp, turn = warp == 0 ? -1 : 0; k < nrec; k += kTriWarps, turn++) {
       if (turn >= 0 && !mbar_wait(&S.turn[warp], turn & 1)) {  // record k - 1 is solved
         atomicExch(err, 1);
@@ -574,7 +566,7 @@ __global__ void __launch_bounds__(kTriThreads) k_ilu_tri(int N, const uint4 *__r
         if (have && (t.flags & 4)) mbar_arrive(&S.empty[ci % kTriStages]);
       }
       have = false;
-      if (k + kTriWarps < nrec) fetch(kTriWarps - 1);
+      if (k + kTriWarps < nrec) fetch();
     }
   }
   __syncthreads();
@@ -784,7 +776,8 @@ static int ilu_apply_dev(exf_sys *s, int lev, const double *c, double *y, const 
   const int N = L.N, G = ilu_grid(s);
   if (L.ilu_nsrc) {  // the streams exist: one CTA
     k_ilu_tri<<<1, kTriThreads, sizeof(TriSmem) + (size_t)(N + 1) * sizeof(double), s->stream>>>(
-        N, L.ilu_str.p, L.ilu_chunk.p, L.ilu_nchunk, L.ilu_nrec[0], L.ilu_nrec[0] + L.ilu_nrec[1], c, y, s->wait_flag.p, skip);
+        N, L.ilu_str.p, L.ilu_chunk.p, L.ilu_nchunk, L.ilu_nrec[0], L.ilu_nrec[0] + L.ilu_nrec[1], L.ilu_first, c, y,
+        s->wait_flag.p, skip);
     EXF_COUNT(1);
     EXF_LAUNCH_CHECK();
     return EXF_OK;
@@ -814,96 +807,24 @@ static int launch_factor(exf_sys *s, SysLevel &L) {
   return EXF_OK;
 }
 
-// The rows in the order their tickets hand them out: by dependency level (the longest
-// chain of lower, or upper, entries leading to the row), index order within a level.
-// Every row depends only on rows of earlier levels, so a warp still waits only on earlier
-// tickets, and the rows of a level run together instead of one index after the other
-// (consecutive rows of the level-nested numbering mostly depend on each other).
-// Returns the number of levels.
-static int level_order(const std::vector<int> &ptr, const std::vector<int> &col, const std::vector<int> &dp,
-                       bool upper, std::vector<int> &ord, std::vector<int> *level = nullptr) {
-  const int N = (int)dp.size();
-  std::vector<int> lv(N, 0);
-  int nl = 0;
-  for (int q = 0; q < N; q++) {
-    const int i = upper ? N - 1 - q : q;
-    int l = 0;
-    const int a = upper ? dp[i] + 1 : ptr[i], e = upper ? ptr[i + 1] : dp[i];
-    for (int k = a; k < e; k++) l = std::max(l, lv[col[k]] + 1);
-    lv[i] = l;
-    nl = std::max(nl, l + 1);
-  }
-  std::vector<int> cnt(nl + 1, 0);
-  for (int i = 0; i < N; i++) cnt[lv[i] + 1]++;
-  for (int l = 0; l < nl; l++) cnt[l + 1] += cnt[l];
-  ord.assign(N, 0);
-  for (int i = 0; i < N; i++) ord[cnt[lv[i]]++] = i;
-  if (level) *level = std::move(lv);
-  return nl;
-}
-
-// The streams of k_ilu_tri for one level, from the pattern (fixed per system): the rows by
-// dependency level, a level's rows longest first, consecutive records packed into chunks
+// The streams of k_ilu_tri for one level, from the pattern (fixed per system)
 static int build_streams(exf_sys *s, SysLevel &L, const std::vector<int> &ptr, const std::vector<int> &col,
                          const std::vector<int> &dp) {
-  const int N = L.N;
-  if (sizeof(TriSmem) + (size_t)(N + 1) * sizeof(double) > kTriSmem) return EXF_OK;
+  if (sizeof(TriSmem) + (size_t)(L.N + 1) * sizeof(double) > kTriSmem) return EXF_OK;
   EXF_CUDA(cudaFuncSetAttribute(k_ilu_tri, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTriSmem));
-  std::vector<uint4> str;
-  std::vector<int2> src, chunk;
-  size_t newest = 0;  // the last record
-  L.ilu_nrec[0] = L.ilu_nrec[1] = 0;
-  for (int up = 0; up < 2; up++) {
-    std::vector<int> ord, lv;
-    level_order(ptr, col, dp, up == 1, ord, &lv);
-    auto len = [&](int i) { return up ? ptr[i + 1] - 1 - dp[i] : dp[i] - ptr[i]; };
-    for (int a = 0; a < N;) {
-      int e = a;
-      while (e < N && lv[ord[e]] == lv[ord[a]]) e++;
-      std::stable_sort(ord.begin() + a, ord.begin() + e, [&](int x, int y) { return len(x) > len(y); });
-      for (; a < e; a += 32) {
-        const int R = std::min(32, e - a), most = len(ord[a]);
-        for (int j0 = 0; j0 == 0 || j0 < most; j0 += kTriE) {
-          const int M = (std::min(kTriE, most - j0) + 3) & ~3, w = tri_words(M);
-          const size_t o = str.size();
-          if (chunk.empty() || chunk.back().y + w > kTriWords) {
-            if (!chunk.empty()) str[newest].y |= 4u;
-            chunk.push_back(make_int2((int)o, 0));
-          }
-          chunk.back().y += w;
-          newest = o;
-          L.ilu_nrec[up]++;
-          str.resize(o + w, make_uint4(0u, 0u, 0u, 0u));
-          str[o] = make_uint4((unsigned)M / 4, (j0 == 0 ? 1u : 0u) | (j0 + kTriE >= most ? 2u : 0u), (unsigned)w, 0u);
-          int *row = reinterpret_cast<int *>(&str[o + 1]), *ix = reinterpret_cast<int *>(&str[o + 41]);
-          for (int k = 0; k < 32; k++) row[k] = N;
-          for (int k = 0; k < 32 * M; k++) ix[k] = N;
-          for (int r = 0; r < R; r++) {
-            const int i = ord[a + r];
-            row[r] = i;
-            src.push_back(make_int2((int)(2 * (o + 9)) + r, ~i));
-            src.push_back(make_int2((int)(2 * (o + 25)) + r, dp[i]));
-            for (int j = j0; j < std::min(len(i), j0 + M); j++) {
-              const int k = up ? ptr[i + 1] - 1 - j : ptr[i] + j;  // upper: from the row's end
-              ix[(j - j0) * 32 + r] = col[k];
-              src.push_back(make_int2((int)(2 * (o + 41 + 8 * M)) + (j - j0) * 32 + r, k));
-            }
-          }
-        }
-      }
-      a = e;
-    }
-  }
-  str[newest].y |= 4u;
-  L.ilu_nchunk = (int)chunk.size();
-  EXF_TRY(L.ilu_str.alloc(str.size()));
-  EXF_TRY(L.ilu_src.alloc(src.size()));
-  EXF_TRY(L.ilu_chunk.alloc(chunk.size()));
-  EXF_CUDA(cudaMemcpyAsync(L.ilu_str.p, str.data(), str.size() * sizeof(uint4), cudaMemcpyHostToDevice, s->stream));
-  EXF_CUDA(cudaMemcpyAsync(L.ilu_src.p, src.data(), src.size() * sizeof(int2), cudaMemcpyHostToDevice, s->stream));
-  EXF_CUDA(cudaMemcpyAsync(L.ilu_chunk.p, chunk.data(), chunk.size() * sizeof(int2), cudaMemcpyHostToDevice, s->stream));
+  const TriStream T = build_tri_stream(ptr, col, dp);
+  EXF_TRY(L.ilu_str.alloc(T.str.size()));
+  EXF_TRY(L.ilu_src.alloc(T.src.size()));
+  EXF_TRY(L.ilu_chunk.alloc(T.chunk.size()));
+  EXF_CUDA(cudaMemcpyAsync(L.ilu_str.p, T.str.data(), T.str.size() * sizeof(uint4), cudaMemcpyHostToDevice, s->stream));
+  EXF_CUDA(cudaMemcpyAsync(L.ilu_src.p, T.src.data(), T.src.size() * sizeof(int2), cudaMemcpyHostToDevice, s->stream));
+  EXF_CUDA(cudaMemcpyAsync(L.ilu_chunk.p, T.chunk.data(), T.chunk.size() * sizeof(int2), cudaMemcpyHostToDevice,
+                           s->stream));
   EXF_CUDA(cudaStreamSynchronize(s->stream));
-  L.ilu_nsrc = (int)src.size();
+  L.ilu_nchunk = (int)T.chunk.size();
+  for (int u = 0; u < 2; u++) L.ilu_nrec[u] = T.nrec[u];
+  L.ilu_first = make_uint4(T.first[0], T.first[1], T.first[2], T.first[3]);
+  L.ilu_nsrc = (int)T.src.size();
   return EXF_OK;
 }
 
