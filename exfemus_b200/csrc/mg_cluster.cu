@@ -67,6 +67,7 @@ struct CluArgs {
   int steps, xlen, mlen;        // most steps of a level, longest iterate, most entries of a CTA
   int *wait_flag;
   T damp;
+  int overwrite;                // correction factor 0: x = P x_c, as prolong_add
   const double *inv;            // coarsest inverse, gauge mask
   const double *gmask;
 };
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(kCluNT, 1) k_mg_cluster(const __grid_constant_
   } else {
     l++;  // CTAs that left the descent rejoin at the lowest level they share
   }
-  // up: x += damp * P x_c, post-smoothing
+  // up: x += damp * P x_c (or x = P x_c), post-smoothing
   bool apart = act1 == 1;  // CTA 0 is on its own
   for (; l <= A.hi; l++) {
     const CluLevel<T> &L = A.lev[l];
@@ -406,7 +407,7 @@ __global__ void __launch_bounds__(kCluNT, 1) k_mg_cluster(const __grid_constant_
       for (int f = gt; f < L.N; f += nth) {
         T acc = T(0);
         for (int k = L.p_ptr[f]; k < L.p_ptr[f + 1]; k++) acc += L.p_val[k] * xc[L.p_col[k]];
-        L.x[f] += A.damp * acc;
+        L.x[f] = A.overwrite ? acc : L.x[f] + A.damp * acc;
       }
       load_level<T, LPR>(L, rank, S);
     }
@@ -633,6 +634,7 @@ int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi, bool zero
   A.reverse = p->reverse_colours ? 1 : 0;
   A.zero_hi = zero_hi ? 1 : 0;
   A.damp = (T)p->corr_damp;
+  A.overwrite = p->corr_damp == 0. ? 1 : 0;
   A.inv = s->coarse_inv.p;
   A.gmask = s->gmask0.p;
   A.wait_flag = s->wait_flag.p;
