@@ -30,11 +30,8 @@
 
 namespace exf {
 
-static constexpr int kCluMaxLev = 10;
 // 512 threads: 256 cost 7% more on the 129 x 129 lattice (rounds of rows), 1024 spill
 static constexpr int kCluNT = 512;
-static constexpr size_t kCluSmem = 224 * 1024;  // dynamic shared memory of a CTA
-static constexpr size_t kCluRep = 152 * 1024;   // of these, the iterate at most
 // lanes per row; a warp's rows are consecutive in colour order, so their new values leave
 // as vectors
 static constexpr int clu_lpr(int dim) { return dim == 2 ? 8 : 16; }
@@ -561,28 +558,25 @@ int build_cluster(exf_sys *s, int lev, const std::vector<int> &items) {
   return EXF_OK;
 }
 
-static size_t cluster_smem(size_t T, int gc, int steps, int xlen, int mlen) {
-  return (size_t)steps * gc * (16 + 2 * T) + (size_t)steps * 8 + (size_t)xlen * T + (size_t)mlen * (4 + T);
+static bool shape_of(const exf_sys *s, int hi, size_t elem, CluShape &S) {
+  return cluster_shape(hi, elem, kCluNT / clu_lpr(s->dim), [&](int l) -> const CluTable & { return s->L[l].clu; }, S);
 }
 
 // whether levels `lev` .. 0 may run in the cluster kernel with values of `elem` bytes
 bool mg_cluster_level(const exf_sys *s, int lev, size_t elem) {
-  if (s->nv1 != 0) return false;
-  for (int l = lev; l >= 1; l--) {
-    const CluTable &C = s->L[l].clu;
-    if (!C.ok || (size_t)C.Np * elem > kCluRep ||
-        cluster_smem(elem, kCluNT / clu_lpr(s->dim), C.steps, C.Np + 3, 0) > kCluSmem)
-      return false;
-  }
-  return true;
+  CluShape S;
+  return s->nv1 == 0 && shape_of(s, lev, elem, S);
 }
 
 // levels hi .. 0 of one V-cycle (gamma 1): x of level hi, from b of level hi
 template <class T>
 int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi, bool zero_hi) {
   CluArgs<T> A = {};
-  const int gc = kCluNT / clu_lpr(s->dim);
-  int want = 1;
+  CluShape S;
+  if (!shape_of(s, hi, sizeof(T), S)) {
+    set_error("level %d does not fit the cluster cycle", hi);
+    return EXF_ERR_UNSUPPORTED;
+  }
   for (int l = hi; l >= 0; l--) {
     SysLevel &L = s->L[l];
     CluLevel<T> &d = A.lev[l];
@@ -595,6 +589,7 @@ int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi, bool zero
     d.steps = L.clu.steps;
     d.exch = L.clu.exch;
     d.act = L.clu.act;
+    d.mat = S.mat[l];
     d.tab = L.clu.tab;
     d.first = L.clu.first;
     d.ent = L.clu.ent;
@@ -610,21 +605,10 @@ int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi, bool zero
     d.p_ptr = L.Pq.ptr.p;
     d.p_col = L.Pq.col.p;
     d.p_val = CV<T>::val(L.Pq);
-    want = std::max(want, d.act);
-    A.steps = std::max(A.steps, d.steps);
-    A.xlen = std::max(A.xlen, (d.Np + 3) & ~3);
   }
-  A.steps = (A.steps + 1) & ~1;  // 16-byte alignment of what follows the steps
-  for (int l = hi; l >= 1; l--) {  // the rows' entries of the levels where they fit beside the tables
-    const int n = s->L[l].clu.entries;
-    A.lev[l].mat = n > 0 && cluster_smem(sizeof(T), gc, A.steps, A.xlen, n) <= kCluSmem ? n : 0;
-    A.mlen = std::max(A.mlen, A.lev[l].mat);
-  }
-  const size_t smem = cluster_smem(sizeof(T), gc, A.steps, A.xlen, A.mlen);
-  if (smem > kCluSmem) {
-    set_error("the cluster cycle needs %zu bytes of shared memory", smem);
-    return EXF_ERR_UNSUPPORTED;
-  }
+  A.steps = S.steps;
+  A.xlen = S.xlen;
+  A.mlen = S.mlen;
   A.hi = hi;
   const int mul = p->double_below_top ? 2 : 1;
   A.nu_pre = p->nu_pre * mul;
@@ -639,13 +623,13 @@ int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi, bool zero
   A.gmask = s->gmask0.p;
   A.wait_flag = s->wait_flag.p;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(want);
+  cfg.gridDim = dim3(S.act);
   cfg.blockDim = dim3(kCluNT);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = S.smem;
   cfg.stream = s->stream;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = want;
+  at[0].val.clusterDim.x = S.act;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;

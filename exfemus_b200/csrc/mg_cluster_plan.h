@@ -1,12 +1,17 @@
 // mg_cluster_plan.h -- which CTA, warp and step of the cluster kernel (mg_cluster.cu) updates
-// which row of a scalar level.  Host code on plain arrays, no CUDA types, so that the rules
+// which row of a scalar level, and which levels fit one launch.  Host code on plain arrays, no CUDA types, so that the rules
 // the kernel's exchange rests on can be checked without a device.
 #pragma once
 #include <algorithm>
+#include <cstddef>
 #include <cstdint>
 #include <vector>
 
 namespace exf {
+
+constexpr int kCluMaxLev = 10;
+constexpr size_t kCluSmem = 224 * 1024;  // dynamic shared memory of a CTA
+constexpr size_t kCluRep = 152 * 1024;   // of these, the iterate at most
 
 struct CluRow {  // a row group's row in one step
   int pos, k0, len, diag;  // position or -1 (none), first entry, entries (0: padding), diagonal - first
@@ -82,6 +87,42 @@ inline CluPlan plan_cluster(int N, const int *qp, const int *diag, int ncolour, 
     P.entries = std::max(P.entries, (at + 3) & ~3);
   }
   return P;
+}
+
+// Dynamic shared memory of a CTA: the step tables (rows, reciprocals, rhs), the steps, the
+// iterate and the copied entries, sized for the largest of a launch's levels each
+constexpr size_t cluster_smem(size_t elem, int gc, int steps, int xlen, int mlen) {
+  return (size_t)steps * gc * (16 + 2 * elem) + (size_t)steps * 8 + (size_t)xlen * elem + (size_t)mlen * (4 + elem);
+}
+
+struct CluShape {
+  int act = 1, steps = 0, xlen = 0, mlen = 0;  // CTAs, most steps, longest iterate, most entries of a CTA
+  int mat[kCluMaxLev] = {0};                   // entries of a CTA in shared memory per level (0: not there)
+  size_t smem = 0;
+};
+// Whether levels hi .. 1 fit one launch with values of `elem` bytes, and its sizes; lev(l)
+// gives a level's ok, act, steps, Np and entries.  Both the choice of the cluster path and
+// the launch use this.  CTAs above 0 leave the descent at the first level of one CTA, so a
+// coarser level must not need more CTAs than a finer one.
+template <class Lev>
+inline bool cluster_shape(int hi, size_t elem, int gc, Lev lev, CluShape &S) {
+  S = CluShape();
+  if (hi < 1 || hi >= kCluMaxLev) return false;
+  for (int l = 1; l <= hi; l++) {
+    const auto &C = lev(l);
+    if (!C.ok || (size_t)C.Np * elem > kCluRep || C.act < S.act) return false;
+    S.act = C.act;
+    S.steps = std::max(S.steps, (C.steps + 1) & ~1);  // 16-byte alignment of what follows the steps
+    S.xlen = std::max(S.xlen, (C.Np + 3) & ~3);
+  }
+  if (cluster_smem(elem, gc, S.steps, S.xlen, 0) > kCluSmem) return false;
+  for (int l = 1; l <= hi; l++) {  // the rows' entries of the levels where they fit beside the tables
+    const int n = lev(l).entries;
+    S.mat[l] = n > 0 && cluster_smem(elem, gc, S.steps, S.xlen, n) <= kCluSmem ? n : 0;
+    S.mlen = std::max(S.mlen, S.mat[l]);
+  }
+  S.smem = cluster_smem(elem, gc, S.steps, S.xlen, S.mlen);
+  return true;
 }
 
 }  // namespace exf

@@ -40,13 +40,17 @@ int main() {
 """
 
 
-@pytest.fixture(scope="module")
-def planner(tmp_path_factory):
+def compile_cpp(d, name):
     if not shutil.which("g++"):
         pytest.skip("no g++")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", CSRC, str(d / (name + ".cpp")), "-o", str(d / name)], check=True)
+
+
+@pytest.fixture(scope="module")
+def planner(tmp_path_factory):
     d = tmp_path_factory.mktemp("plan")
     (d / "plan.cpp").write_text(PROGRAM)
-    subprocess.run(["g++", "-std=c++17", "-O1", "-I", CSRC, str(d / "plan.cpp"), "-o", str(d / "plan")], check=True)
+    compile_cpp(d, "plan")
 
     def run(colour, length, lpr):
         nc = int(colour.max()) + 1
@@ -221,3 +225,45 @@ def test_the_model_sees_a_missing_unit_and_a_missing_arrival(planner):
     bare[6:, 14:] = 0  # the last line class has 14 warps of rows
     assert any(exchange(bare, 2, random.Random(s)) for s in range(20))
     assert any(exchange(u, 2, random.Random(s), all_warps_arrive=False) for s in range(20))
+
+
+SHAPE = r"""
+#include <cstdio>
+#include "mg_cluster_plan.h"
+struct Lev { int ok, act, steps, Np, entries; };
+int main() {
+  int hi, elem, gc;
+  if (scanf("%d %d %d", &hi, &elem, &gc) != 3) return 1;
+  std::vector<Lev> L(hi + 1);
+  for (int l = 1; l <= hi; l++)
+    if (scanf("%d %d %d %d %d", &L[l].ok, &L[l].act, &L[l].steps, &L[l].Np, &L[l].entries) != 5) return 1;
+  exf::CluShape S;
+  const bool ok = exf::cluster_shape(hi, elem, gc, [&](int l) -> const Lev & { return L[l]; }, S);
+  printf("%d %d %d %d %d %zu", ok, S.act, S.steps, S.xlen, S.mlen, S.smem);
+  for (int l = 1; l <= hi && l < exf::kCluMaxLev; l++) printf(" %d", S.mat[l]);
+}
+"""
+
+
+def test_levels_of_a_launch(tmp_path):
+    """Levels that fit alone but not together, and a coarse level of more CTAs than the next."""
+    (tmp_path / "shape.cpp").write_text(SHAPE)
+    compile_cpp(tmp_path, "shape")
+
+    def shape(levels, elem=8, gc=64):
+        text = "%d %d %d\n" % (len(levels), elem, gc) + "\n".join("%d %d %d %d %d" % lev for lev in levels)
+        out = subprocess.run([str(tmp_path / "shape")], input=text, capture_output=True, text=True, check=True)
+        v = [int(x) for x in out.stdout.split()]
+        return bool(v[0]), dict(act=v[1], steps=v[2], xlen=v[3], mlen=v[4], smem=v[5], mat=v[6:])
+
+    smem = lambda steps, xlen, mlen: steps * 64 * 32 + steps * 8 + xlen * 8 + mlen * 12  # noqa: E731
+    ok, s = shape([(1, 1, 9, 81, 1000), (1, 16, 9, 2000, 900), (1, 16, 27, 17001, 0)])
+    assert ok and s["act"] == 16 and s["steps"] == 28 and s["xlen"] == 17004
+    assert s["mat"] == [1000, 900, 0] and s["mlen"] == 1000 and s["smem"] == smem(28, 17004, 1000) <= 224 * 1024
+    many_steps, long = (1, 16, 60, 2000, 0), (1, 16, 9, 19000, 0)
+    assert shape([many_steps])[0] and shape([(1, 16, 9, 2000, 0), long])[0]
+    assert smem(60, 19000, 0) > 224 * 1024 and not shape([many_steps, long])[0]
+    # an odd step count at the limit is rounded up before it is compared
+    assert smem(41, 18132, 0) <= 224 * 1024 < smem(42, 18132, 0) and not shape([(1, 16, 41, 18132, 0)])[0]
+    assert not shape([(1, 16, 9, 500, 0), (1, 1, 9, 600, 0)])[0]
+    assert not shape([(0, 1, 9, 81, 0)])[0] and not shape([(1, 1, 9, 81, 0)] * 10)[0]
