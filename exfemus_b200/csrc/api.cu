@@ -262,7 +262,7 @@ static int mg_step(exf_sys *s, int lev, const exf_mg_params *p, bool final_resid
   // Gauss-Seidel levels that fit a cluster: this level and all below it in one launch
   if (p->smoother == EXF_SMOOTH_GS && p->gamma == 1 && !acc && mg_cluster_level(s, lev, sizeof(T))) {
     if (!s->coarse_ok) EXF_TRY(coarse_factor(s));
-    EXF_TRY(mg_cluster<T>(s, lev, p, mul, false));
+    EXF_TRY(mg_cluster<T>(s, lev, p, mul));
     if (final_resid) EXF_TRY(spmv_resid<T>(s, lev, x, b, r, d_norm_out));
     return EXF_OK;
   }

@@ -450,7 +450,7 @@ int smooth(exf_sys *s, int lev, const exf_mg_params *p, int nsweeps, T *x, const
 int build_cluster(exf_sys *s, int lev, const std::vector<int> &items);
 bool mg_cluster_level(const exf_sys *s, int lev, size_t elem);
 template <class T>
-int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi, bool zero_hi);
+int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi);
 // EXF_ERR_CUDA (and clears the flag) when a bounded in-kernel wait ran out since the last call
 int device_wait_status(exf_sys *s);
 // GMRES + ILU level solver (ilu_gmres.cu)

@@ -60,7 +60,7 @@ struct CluArgs {
   int hi;                       // levels hi .. 1 are smoothed
   int nu_pre, nu_post;          // sweeps of a level below the top
   int nu_pre_hi, nu_post_hi;    // sweeps of level hi
-  int reverse, zero_hi;         // zero_hi: level hi starts from x = 0
+  int reverse;
   int steps, xlen, mlen;        // most steps of a level, longest iterate, most entries of a CTA
   int *wait_flag;
   T damp;
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(kCluNT, 1) k_mg_cluster(const __grid_constant_
     const int nth = L.act * kCluNT, gt = rank * kCluNT + tid;
     if (in) {
       load_level<T, LPR>(L, rank, S);
-      fill_x(L, l < A.hi || A.zero_hi, S);
+      fill_x(L, l < A.hi, S);
     }
     phase_sync(L.act);
     if (in) {
@@ -570,7 +570,7 @@ bool mg_cluster_level(const exf_sys *s, int lev, size_t elem) {
 
 // levels hi .. 0 of one V-cycle (gamma 1): x of level hi, from b of level hi
 template <class T>
-int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi, bool zero_hi) {
+int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi) {
   CluArgs<T> A = {};
   CluShape S;
   if (!shape_of(s, hi, sizeof(T), S)) {
@@ -616,7 +616,6 @@ int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi, bool zero
   A.nu_pre_hi = p->nu_pre * mul_hi;
   A.nu_post_hi = p->nu_post * mul_hi;
   A.reverse = p->reverse_colours ? 1 : 0;
-  A.zero_hi = zero_hi ? 1 : 0;
   A.damp = (T)p->corr_damp;
   A.overwrite = p->corr_damp == 0. ? 1 : 0;
   A.inv = s->coarse_inv.p;
@@ -639,7 +638,7 @@ int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi, bool zero
   EXF_COUNT(1);
   return EXF_OK;
 }
-template int mg_cluster<double>(exf_sys *, int, const exf_mg_params *, int, bool);
-template int mg_cluster<float>(exf_sys *, int, const exf_mg_params *, int, bool);
+template int mg_cluster<double>(exf_sys *, int, const exf_mg_params *, int);
+template int mg_cluster<float>(exf_sys *, int, const exf_mg_params *, int);
 
 }  // namespace exf
