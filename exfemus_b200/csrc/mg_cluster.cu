@@ -32,6 +32,12 @@ namespace exf {
 
 // 512 threads: 256 cost 7% more on the 129 x 129 lattice (rounds of rows), 1024 spill
 static constexpr int kCluNT = 512;
+// Rows of the coarsest level up to which its product runs in the cluster.  It reads n^2
+// doubles through at most 16 SMs; above, the descent and the ascent are two launches around
+// the product on all SMs.  Two-level V-cycle with one pre- and post-sweep, in one launch and
+// in three (FP64, us): n = 289 39 and 41, 625 43 and 42, 729 (3D) 102 and 102, 1225 56 and
+// 52, 2401 113 and 78, 4761 645 and 172 (FP32 9801: 2186 and 429).
+static constexpr int kCluCoarse = 700;
 // lanes per row; a warp's rows are consecutive in colour order, so their new values leave
 // as vectors
 static constexpr int clu_lpr(int dim) { return dim == 2 ? 8 : 16; }
@@ -61,6 +67,7 @@ struct CluArgs {
   int nu_pre, nu_post;          // sweeps of a level below the top
   int nu_pre_hi, nu_post_hi;    // sweeps of level hi
   int reverse;
+  int part;                     // 1: descent, 2: coarsest product, 4: ascent
   int steps, xlen, mlen;        // most steps of a level, longest iterate, most entries of a CTA
   int *wait_flag;
   T damp;
@@ -328,7 +335,12 @@ __global__ void __launch_bounds__(kCluNT, 1) k_mg_cluster(const __grid_constant_
   // A level's work is done by its first `act` CTAs; with act == 1 the others are not even at
   // its barriers.  down: x = 0 (or given), pre-smoothing, residual, restriction
   int l = A.hi;
-  for (; l >= 1; l--) {
+  if (!(A.part & 1)) {  // the ascent alone: where the descent ends
+    l = 0;
+    if (rank > 0)
+      while (l < A.hi && A.lev[l + 1].act == 1) l++;
+  }
+  for (; (A.part & 1) && l >= 1; l--) {
     const CluLevel<T> &L = A.lev[l];
     if (L.act == 1 && rank > 0) break;  // the levels from here down belong to CTA 0
     const bool in = rank < L.act;
@@ -372,7 +384,7 @@ __global__ void __launch_bounds__(kCluNT, 1) k_mg_cluster(const __grid_constant_
   }
   // coarsest level: x = A0^{-1} (b * gmask), a warp per row
   const int act1 = A.lev[1].act;
-  if (l == 0) {
+  if (l == 0 && (A.part & 2)) {
     const CluLevel<T> &L = A.lev[0];
     const int n = L.N, w = (rank * kCluNT + tid) >> 5, wl = tid & 31;
     const int nw = (act1 == 1 ? 1 : csize) * (kCluNT / 32);
@@ -384,10 +396,9 @@ __global__ void __launch_bounds__(kCluNT, 1) k_mg_cluster(const __grid_constant_
       if (wl == 0) L.x[row] = (T)acc;
     }
     phase_sync(act1);
-    l = 1;
-  } else {
-    l++;  // CTAs that left the descent rejoin at the lowest level they share
   }
+  if (!(A.part & 4)) return;
+  l++;  // CTAs that left the descent rejoin at the lowest level they share
   // up: x += damp * P x_c (or x = P x_c), post-smoothing
   bool apart = act1 == 1;  // CTA 0 is on its own
   for (; l <= A.hi; l++) {
@@ -568,7 +579,8 @@ bool mg_cluster_level(const exf_sys *s, int lev, size_t elem) {
   return s->nv1 == 0 && shape_of(s, lev, elem, S);
 }
 
-// levels hi .. 0 of one V-cycle (gamma 1): x of level hi, from b of level hi
+// levels hi .. 0 of one V-cycle (gamma 1): x of level hi, from b of level hi; one launch, or
+// three with a large coarsest level
 template <class T>
 int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi) {
   CluArgs<T> A = {};
@@ -634,8 +646,18 @@ int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi) {
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
+  if (s->L[0].N <= kCluCoarse) {
+    A.part = 7;
+    EXF_CUDA(cudaLaunchKernelEx(&cfg, cluster_kernel<T>(s->dim), A));
+    EXF_COUNT(1);
+    return EXF_OK;
+  }
+  A.part = 1;
   EXF_CUDA(cudaLaunchKernelEx(&cfg, cluster_kernel<T>(s->dim), A));
-  EXF_COUNT(1);
+  EXF_TRY(coarse_apply<T>(s, A.lev[0].b, A.lev[0].x));
+  A.part = 4;
+  EXF_CUDA(cudaLaunchKernelEx(&cfg, cluster_kernel<T>(s->dim), A));
+  EXF_COUNT(2);
   return EXF_OK;
 }
 template int mg_cluster<double>(exf_sys *, int, const exf_mg_params *, int);

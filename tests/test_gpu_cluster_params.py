@@ -41,3 +41,29 @@ def test_correction_factor(gpu_lib, dim, nlev, n0, damp):
     t.solve(p)
     # a cycle is a few thousand roundings of 1.1e-16 in operators whose sweeps contract
     assert rel(t.x(), compose(t, p, nlev - 1, x0, t.rhs())) <= 1e-12
+
+
+@pytest.mark.parametrize("dim,n0", [(2, (12, 13)), (2, (13, 13)), (2, (24, 5)), (3, (4, 4, 4)), (3, (5, 3, 4))])
+def test_coarsest_product_inside_and_outside_the_launch(gpu_lib, dim, n0):
+    """Coarsest levels on either side of the line at 700 rows: 675, 729, 539, 729 and 693."""
+    m = ex.Mesh(dim, 2, n0, (0, 2, 0, 1, 0, 1)[:2 * dim])
+    t = ex.MGSolT(m)
+    t.GenBc(_lib.BC_HEAT_DIRICHLET)
+    t.phys = ex.phys(inv_dt=3.0)
+    rng = np.random.default_rng(n0[0])
+    t.set_source(workloads.heat_source(m.nel(1)))
+    t.set_xold(rng.standard_normal(t.ntop_dof))
+    t.assemble_all()
+    x0 = rng.standard_normal(t.ntop_dof)
+    p = ex.mg_params(max_cycles=1, eps=1e-30)
+    t.set_x(x0)
+    t.solve(p)
+    one = t.x()
+    # a cycle is a few thousand roundings of 1.1e-16 in operators whose sweeps contract
+    assert rel(one, compose(t, p, 1, x0, t.rhs())) <= 1e-12
+    outs = []
+    for graph in (0, 1):
+        t.set_x(x0)
+        t.solve(ex.mg_params(max_cycles=3, eps=1e-30, use_graph=graph))
+        outs.append(t.x())
+    assert np.array_equal(outs[0], outs[1])
