@@ -260,7 +260,8 @@ static int mg_step(exf_sys *s, int lev, const exf_mg_params *p, bool final_resid
   }
   const int mul = (p->double_below_top && lev < top) ? 2 : 1;
   // Gauss-Seidel levels that fit a cluster: this level and all below it in one launch
-  if (p->smoother == EXF_SMOOTH_GS && p->gamma == 1 && !acc && mg_cluster_level(s, lev, sizeof(T))) {
+  if (p->smoother == EXF_SMOOTH_GS && p->gamma == 1 && !acc &&
+      mg_cluster_level(s, lev, sizeof(T), (p->nu_pre + p->nu_post) * mul)) {
     if (!s->coarse_ok) EXF_TRY(coarse_factor(s));
     EXF_TRY(mg_cluster<T>(s, lev, p, mul));
     if (final_resid) EXF_TRY(spmv_resid<T>(s, lev, x, b, r, d_norm_out));

@@ -448,7 +448,7 @@ template <class T>
 int smooth(exf_sys *s, int lev, const exf_mg_params *p, int nsweeps, T *x, const T *b);
 // levels hi .. 0 of a scalar system's V-cycle in one cluster launch (mg_cluster.cu)
 int build_cluster(exf_sys *s, int lev, const std::vector<int> &items);
-bool mg_cluster_level(const exf_sys *s, int lev, size_t elem);
+bool mg_cluster_level(const exf_sys *s, int lev, size_t elem, int sweeps);
 template <class T>
 int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi);
 // EXF_ERR_CUDA (and clears the flag) when a bounded in-kernel wait ran out since the last call

@@ -573,10 +573,11 @@ static bool shape_of(const exf_sys *s, int hi, size_t elem, CluShape &S) {
   return cluster_shape(hi, elem, kCluNT / clu_lpr(s->dim), [&](int l) -> const CluTable & { return s->L[l].clu; }, S);
 }
 
-// whether levels `lev` .. 0 may run in the cluster kernel with values of `elem` bytes
-bool mg_cluster_level(const exf_sys *s, int lev, size_t elem) {
+// whether levels `lev` .. 0 run in the cluster kernel with values of `elem` bytes, level lev
+// with `sweeps` sweeps per cycle
+bool mg_cluster_level(const exf_sys *s, int lev, size_t elem, int sweeps) {
   CluShape S;
-  return s->nv1 == 0 && shape_of(s, lev, elem, S);
+  return s->nv1 == 0 && s->L[lev].N <= cluster_rows(s->dim, sweeps) && shape_of(s, lev, elem, S);
 }
 
 // levels hi .. 0 of one V-cycle (gamma 1): x of level hi, from b of level hi; one launch, or

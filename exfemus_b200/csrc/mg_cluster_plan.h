@@ -89,6 +89,23 @@ inline CluPlan plan_cluster(int N, const int *qp, const int *diag, int ncolour, 
   return P;
 }
 
+// Most rows of a level that is faster in the cluster than with a launch per colour, with
+// `sweeps` sweeps per cycle.  A sweep in the cluster grows with the rows (16 SMs) while
+// launches cost the same up to here, and the restriction, prolongation and residual that go
+// with the level lose from the start.  V-cycle down from such a level, cluster and launches
+// (us): 2D FP64 9,409 rows 2 sweeps 125 and 127, 12,769 rows 2 sweeps 137 and 129, 4 sweeps
+// 191 and 195, 16,641 rows 8 sweeps 336 and 332, 12 sweeps 456 and 465; FP32 16,641 rows 4
+// sweeps 187 and 178, 8 sweeps 279 and 293, 25,921 rows 12 sweeps 474 and 417; 6,561 rows 1
+// sweep 91 and 94, 0 sweeps 73 and 64.  3D FP32 18,785 rows 2 sweeps 245 and 242, 25,625 rows
+// 4 sweeps 393 and 406, 30,625 rows 8 sweeps 792 and 732; FP64 18,785 rows 1 sweep 207 and
+// 200, 2 sweeps 285 and 308.
+constexpr int cluster_rows(int dim, int sweeps) {
+  return sweeps < 1    ? 0
+         : dim == 3    ? 26000 - 14000 / sweeps
+         : sweeps == 1 ? 6600
+                       : 18300 - 18000 / sweeps;
+}
+
 // Dynamic shared memory of a CTA: the step tables (rows, reciprocals, rhs), the steps, the
 // iterate and the copied entries, sized for the largest of a launch's levels each
 constexpr size_t cluster_smem(size_t elem, int gc, int steps, int xlen, int mlen) {
