@@ -1223,6 +1223,7 @@ int exf_mg_solve(exf_sys *s, const exf_mg_params *p, exf_solve_stats *st) {
     }
     for (int l = p->coarse_iters > 0 ? 0 : 1; l < s->nlev; l++) EXF_TRY(ilu_ready(s, l));  // once per assembly
   }
+  if (p->smoother == EXF_SMOOTH_GS) EXF_TRY(cluster_ready(s));
   if (!s->coarse_ok) EXF_TRY(coarse_factor(s));
   EXF_CUDA(cudaEventRecord(s->ev0, s->stream));
   EXF_TRY(norm2(s, T.b.p, T.ndof, dnb));
@@ -1419,6 +1420,7 @@ int exf_time_op(exf_sys *s, int what, int lev, const exf_mg_params *p, const exf
   if (what == 2 && !ph) return EXF_ERR_ARG;
   if (what != 2 && !s->assembled) return EXF_ERR_STATE;
   if (what == 3) EXF_TRY(need_transfers(s));
+  if (what == 3 && p->smoother == EXF_SMOOTH_GS) EXF_TRY(cluster_ready(s));
   if (!s->coarse_ok && what == 3) EXF_TRY(coarse_factor(s));
   SysLevel &L = s->L[lev];
   const bool f32 = p->precision == EXF_PREC_MIXED;

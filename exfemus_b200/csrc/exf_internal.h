@@ -188,7 +188,6 @@ struct CluTable {
   int act = 1, steps = 0, exch = 0, Np = 0, entries = 0;  // CTAs, steps and exchanges of a sweep, positions,
                                                           // most entries of a CTA (0: too many for its
                                                           // shared memory)
-  DBuf<int4> mem;    // the tables below, behind one another
   const int4 *tab = nullptr;   // [act][steps][groups] {position or -1, first entry, entries (0: padding), diagonal - first}
   const int *first = nullptr;  // [act][steps][groups] first of the row's entries in the CTA's copy
   const int2 *ent = nullptr;   // [act][entries] the copy's entries: {entry of the matrix, position of its column}
@@ -355,6 +354,8 @@ struct exf_sys {
   // exf_assemble_all: per colour the {level, element} work list of every level (top level
   // first) and the levels' argument blocks
   exf::DBuf<unsigned char> asm_work, asm_args;
+  bool clu_ready = false;       // the levels' cluster tables were made, in clu_mem
+  exf::DBuf<int4> clu_mem;
   exf::DBuf<double> resid_vec;  // exf_resid's x, b and r
   std::mutex resid_mu;          // held while a call uses them
   std::vector<int> asm_work_off;
@@ -447,7 +448,7 @@ int prolong_add(exf_sys *s, int lev_f, const T *x_c, T *x_f, double damp);
 template <class T>
 int smooth(exf_sys *s, int lev, const exf_mg_params *p, int nsweeps, T *x, const T *b);
 // levels hi .. 0 of a scalar system's V-cycle in one cluster launch (mg_cluster.cu)
-int build_cluster(exf_sys *s, int lev, const std::vector<int> &items);
+int cluster_ready(exf_sys *s);  // their tables, once per system (outside graph capture)
 bool mg_cluster_level(const exf_sys *s, int lev, size_t elem, int sweeps);
 template <class T>
 int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi);

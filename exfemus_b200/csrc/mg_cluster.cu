@@ -500,14 +500,17 @@ __global__ void k_clu_entries(const int4 *tab, const int *first, int ntab, int p
   for (int i = threadIdx.x % 8; i < d.z; i += 8) o[i] = make_int2(d.y + i, col[d.y + i]);
 }
 
-// Tables of a scalar level for the cluster kernel, once per system (plan_cluster)
-int build_cluster(exf_sys *s, int lev, const std::vector<int> &items) {
-  SysLevel &L = s->L[lev];
-  CluTable &C = L.clu;
-  C = CluTable();
-  if (lev == 0 || lev >= kCluMaxLev || (size_t)L.N * sizeof(float) > kCluRep) return EXF_OK;
+// Tables of a scalar system's levels for the cluster kernel (plan_cluster), at its first
+// Gauss-Seidel solve, so that systems solved otherwise do not pay for them: the patterns of
+// all candidate levels in one download, all tables in one block of device memory.  Levels
+// without tables (no cluster on the device, no memory) keep a launch per colour.
+int cluster_ready(exf_sys *s) {
+  if (s->clu_ready) return EXF_OK;
+  s->clu_ready = true;
   const int dev = s->mesh->device;
-  if (dev < 0 || dev >= 64) return EXF_OK;
+  int hi = 0;
+  while (hi + 1 < s->nlev && hi + 1 < kCluMaxLev && s->L[hi + 1].N <= cluster_rows(s->dim, 1 << 20)) hi++;
+  if (s->nv1 != 0 || hi < 1 || dev < 0 || dev >= 64) return EXF_OK;
   static std::atomic<int> fit[2][64];  // per dimension and device: cluster size + 1
   int most = fit[s->dim == 2][dev].load(std::memory_order_acquire) - 1;
   if (most < 0) {
@@ -515,22 +518,20 @@ int build_cluster(exf_sys *s, int lev, const std::vector<int> &items) {
     fit[s->dim == 2][dev].store(most + 1, std::memory_order_release);
   }
   if (most < 1) return EXF_OK;
-  std::vector<int> qp(L.N + 1), diag(L.N);
-  EXF_CUDA(cudaMemcpyAsync(qp.data(), L.qq_ptr.p, qp.size() * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-  EXF_CUDA(cudaMemcpyAsync(diag.data(), L.diag_pos.p, diag.size() * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  std::vector<std::vector<int>> qp(hi + 1), diag(hi + 1), items(hi + 1);
+  for (int l = 1; l <= hi; l++) {
+    SysLevel &L = s->L[l];
+    qp[l].resize(L.N + 1);
+    diag[l].resize(L.N);
+    items[l].resize(L.N);
+    EXF_CUDA(cudaMemcpyAsync(qp[l].data(), L.qq_ptr.p, (L.N + 1) * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    EXF_CUDA(cudaMemcpyAsync(diag[l].data(), L.diag_pos.p, L.N * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    EXF_CUDA(cudaMemcpyAsync(items[l].data(), L.col_items.p, L.N * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  }
   EXF_CUDA(cudaStreamSynchronize(s->stream));
   const int lpr = clu_lpr(s->dim), gc = kCluNT / lpr;
-  const CluPlan P = plan_cluster(L.N, qp.data(), diag.data(), L.ncolour, L.col_off.data(), items.data(), lpr, kCluNT,
-                                 most);
-  C.act = P.act;
-  C.Np = (int)P.node.size();
-  C.steps = (int)P.step.size();
-  C.exch = P.exch;
-  C.entries = P.entries;
-  // entries that fit no CTA's shared memory are read from the level's arrays
-  if ((size_t)C.entries * (4 + sizeof(float)) > kCluSmem) C.entries = 0;
-  // one block of device memory, each table 16-byte aligned: tab, first, step, node, the
-  // node's positions, the columns' positions and the CTAs' entries (these two filled here)
+  // each table 16-byte aligned: tab, first, step, node and the nodes' positions of every
+  // level, then the columns' positions and the CTAs' entries (filled on the device)
   std::vector<int4> mem;
   auto put = [&](const auto &h) {
     const size_t at = mem.size(), bytes = h.size() * sizeof(h[0]);
@@ -539,33 +540,58 @@ int build_cluster(exf_sys *s, int lev, const std::vector<int> &items) {
     return at;
   };
   static_assert(sizeof(CluRow) == sizeof(int4) && sizeof(CluStep) == sizeof(int2), "tables are copied as they are");
-  const size_t o_tab = put(P.tab), o_first = put(P.first), o_step = put(P.step), o_node = put(P.node),
-               o_pos = put(P.pos);
-  const size_t o_col = mem.size(), o_ent = o_col + ((size_t)L.nqq + 3) / 4;
-  EXF_TRY(C.mem.alloc(o_ent + (size_t)C.act * C.entries / 2));
-  EXF_CUDA(cudaMemcpyAsync(C.mem.p, mem.data(), mem.size() * sizeof(int4), cudaMemcpyHostToDevice, s->stream));
-  int *col = reinterpret_cast<int *>(C.mem.p + o_col);
-  int2 *ent = reinterpret_cast<int2 *>(C.mem.p + o_ent);
-  C.tab = C.mem.p + o_tab;
-  C.first = reinterpret_cast<const int *>(C.mem.p + o_first);
-  C.step = reinterpret_cast<const int2 *>(C.mem.p + o_step);
-  C.node = reinterpret_cast<const int *>(C.mem.p + o_node);
-  C.col = col;
-  C.ent = ent;
-  k_clu_columns<<<(unsigned)((L.nqq + 255) / 256), 256, 0, s->stream>>>(
-      L.qq_col.p, reinterpret_cast<const int *>(C.mem.p + o_pos), L.nqq, col);
-  EXF_COUNT(1);
-  if (C.entries) {
-    const int n = C.steps * gc;
-    // every CTA copies C.entries entries: those beyond its rows are entry 0
-    EXF_CUDA(cudaMemsetAsync(ent, 0, (size_t)C.act * C.entries * sizeof(int2), s->stream));
-    k_clu_entries<<<(unsigned)(((long)C.act * n * 8 + 255) / 256), 256, 0, s->stream>>>(C.tab, C.first, C.act * n, n,
-                                                                                       C.entries, col, ent);
+  struct At {
+    size_t tab, first, step, node, pos, col, ent;
+  };
+  std::vector<At> at(hi + 1);
+  for (int l = 1; l <= hi; l++) {
+    SysLevel &L = s->L[l];
+    CluTable &C = L.clu;
+    const CluPlan P = plan_cluster(L.N, qp[l].data(), diag[l].data(), L.ncolour, L.col_off.data(), items[l].data(), lpr,
+                                   kCluNT, most);
+    C.act = P.act;
+    C.Np = (int)P.node.size();
+    C.steps = (int)P.step.size();
+    C.exch = P.exch;
+    // entries that fit no CTA's shared memory are read from the level's arrays
+    C.entries = (size_t)P.entries * (4 + sizeof(float)) > kCluSmem ? 0 : P.entries;
+    at[l] = {put(P.tab), put(P.first), put(P.step), put(P.node), put(P.pos), 0, 0};
+  }
+  size_t len = mem.size();
+  for (int l = 1; l <= hi; l++) {
+    at[l].col = len;
+    at[l].ent = at[l].col + ((size_t)s->L[l].nqq + 3) / 4;
+    len = at[l].ent + (size_t)s->L[l].clu.act * s->L[l].clu.entries / 2;
+  }
+  if (s->clu_mem.alloc(len) != EXF_OK) return EXF_OK;
+  int4 *d = s->clu_mem.p;
+  EXF_CUDA(cudaMemcpyAsync(d, mem.data(), mem.size() * sizeof(int4), cudaMemcpyHostToDevice, s->stream));
+  // every CTA copies C.entries entries: those beyond its rows are entry 0
+  EXF_CUDA(cudaMemsetAsync(d + mem.size(), 0, (len - mem.size()) * sizeof(int4), s->stream));
+  for (int l = 1; l <= hi; l++) {
+    SysLevel &L = s->L[l];
+    CluTable &C = L.clu;
+    int *col = reinterpret_cast<int *>(d + at[l].col);
+    int2 *ent = reinterpret_cast<int2 *>(d + at[l].ent);
+    C.tab = d + at[l].tab;
+    C.first = reinterpret_cast<const int *>(d + at[l].first);
+    C.step = reinterpret_cast<const int2 *>(d + at[l].step);
+    C.node = reinterpret_cast<const int *>(d + at[l].node);
+    C.col = col;
+    C.ent = ent;
+    k_clu_columns<<<(unsigned)((L.nqq + 255) / 256), 256, 0, s->stream>>>(
+        L.qq_col.p, reinterpret_cast<const int *>(d + at[l].pos), L.nqq, col);
     EXF_COUNT(1);
+    if (C.entries) {
+      const int n = C.steps * gc;
+      k_clu_entries<<<(unsigned)(((long)C.act * n * 8 + 255) / 256), 256, 0, s->stream>>>(C.tab, C.first, C.act * n, n,
+                                                                                         C.entries, col, ent);
+      EXF_COUNT(1);
+    }
   }
   EXF_LAUNCH_CHECK();
   EXF_CUDA(cudaStreamSynchronize(s->stream));
-  C.ok = true;
+  for (int l = 1; l <= hi; l++) s->L[l].clu.ok = true;
   return EXF_OK;
 }
 

@@ -47,17 +47,27 @@ inline CluPlan plan_cluster(int N, const int *qp, const int *diag, int ncolour, 
   // exchange), otherwise the whole cluster (just enough CTAs for the rows: 2-6% slower)
   P.act = rows <= gc ? 1 : most;
   P.pos.assign(N, -1);
-  std::vector<int> cbase(ncolour), rounds(ncolour), units(ncolour);
+  int longest = 0;
+  for (int i = 0; i < N; i++) longest = std::max(longest, qp[i + 1] - qp[i]);
+  std::vector<int> cbase(ncolour), rounds(ncolour), units(ncolour), at(longest + 1);
   for (int c = 0; c < ncolour; c++) {
     const int n = col_off[c + 1] - col_off[c];
     units[c] = (n + rw - 1) / rw;
     if (n > 0 && P.act > 1) units[c] = std::max(units[c], P.act);
-    std::vector<int> r(items + col_off[c], items + col_off[c + 1]);
-    std::stable_sort(r.begin(), r.end(), [&](int a, int b) { return qp[a + 1] - qp[a] > qp[b + 1] - qp[b]; });
     cbase[c] = (int)P.node.size();
-    for (int k = 0; k < units[c] * rw; k++) {
-      if (k < n) P.pos[r[k]] = (int)P.node.size();
-      P.node.push_back(k < n ? r[k] : -1);
+    P.node.resize(cbase[c] + units[c] * rw, -1);
+    // longest rows first, rows of one length in the items' order
+    std::fill(at.begin(), at.end(), 0);
+    for (const int *v = items + col_off[c]; v != items + col_off[c + 1]; v++) at[qp[*v + 1] - qp[*v]]++;
+    for (int len = longest, p = cbase[c]; len >= 0; len--) {
+      const int k = at[len];
+      at[len] = p;
+      p += k;
+    }
+    for (const int *v = items + col_off[c]; v != items + col_off[c + 1]; v++) {
+      const int p = at[qp[*v + 1] - qp[*v]]++;
+      P.node[p] = *v;
+      P.pos[*v] = p;
     }
     rounds[c] = (units[c] + P.act * nw - 1) / (P.act * nw);
     for (int k = 0; k < rounds[c]; k++)
@@ -68,12 +78,18 @@ inline CluPlan plan_cluster(int N, const int *qp, const int *diag, int ncolour, 
   P.tab.assign((size_t)P.act * steps * gc, CluRow{-1, 0, 0, -1});
   int st0 = 0;
   for (int c = 0; c < ncolour; c++) {
-    for (int k = 0; k < units[c] * rw; k++) {
-      const int u = k / rw, cta = u % P.act, w = (u / P.act) % nw, rnd = u / P.act / nw;
-      const int p = cbase[c] + k, v = P.node[p];
-      CluRow &t = P.tab[((size_t)cta * steps + st0 + rnd) * gc + w * rw + k % rw];
-      if (v >= 0) t = {p, qp[v], qp[v + 1] - qp[v], diag[v] - qp[v]};
-      else if (k % rw == 0) t = {p, 0, 0, -1};  // a unit of padding: it sends, nothing reads it
+    int cta = 0, slot = st0 * gc;  // of the unit: slot = step, warp and group
+    for (int u = 0, p = cbase[c]; u < units[c]; u++) {
+      CluRow *t = &P.tab[(size_t)cta * steps * gc + slot];
+      for (int g = 0; g < rw; g++, p++) {
+        const int v = P.node[p];
+        if (v >= 0) t[g] = {p, qp[v], qp[v + 1] - qp[v], diag[v] - qp[v]};
+        else if (g == 0) t[g] = {p, 0, 0, -1};  // a unit of padding: it sends, nothing reads it
+      }
+      if (++cta == P.act) {
+        cta = 0;
+        slot += rw;
+      }
     }
     st0 += rounds[c];
   }

@@ -432,7 +432,6 @@ int build_colours(exf_sys *s) {
       EXF_TRY(L.gsrow.alloc(nitem));
       k_gs_rows<<<nblk(nitem, 256), 256, 0, st>>>(L.col_items.p, nitem, L.qq_ptr.p, L.diag_pos.p, L.gsrow.p);
       EXF_LAUNCH_CHECK();
-      EXF_TRY(build_cluster(s, l, items));
     }
     EXF_CUDA(cudaStreamSynchronize(st));
     if (s->kind == EXF_KIND_NS) {
