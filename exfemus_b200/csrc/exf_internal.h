@@ -265,14 +265,14 @@ struct SysLevel {
   DBuf<double> ilu_f, ilu_inv;
   DBuf<int> ilu_flag, ilu_ctl;
   DBuf<int> ilu_ord_lo, ilu_ord_up;  // rows by dependency level of the lower / upper solve
-  // levels whose iterate fits one CTA's shared memory: the factor's entries as two streams
+  // levels solved by one CTA (its shared memory, tri_one_cta): the factor's entries as two streams
   // of records by dependency level (lower, then upper solve), refreshed after each
   // factorisation from {position, source} pairs (ilu_gmres.cu, k_ilu_tri)
   DBuf<uint4> ilu_str;
   DBuf<int2> ilu_src, ilu_chunk;
   int ilu_nsrc = 0, ilu_nchunk = 0, ilu_nrec[2] = {0, 0};
   uint4 ilu_first = {0u, 0u, 0u, 0u};  // places of the first records
-  // levels whose rows have at most kFacMax entries up to the diagonal: the rows of the
+  // levels factored by one CTA (kFacMax entries up to the diagonal, fac_one_cta): the rows of the
   // dense blocks of the factorisation, {entry, place} (k_ilu_struct), and the level offsets
   DBuf<int2> ilu_ent;
   DBuf<int4> ilu_row;

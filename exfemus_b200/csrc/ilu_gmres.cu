@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(32 * NW) k_ilu_factor(int N, const int *__rest
 }
 
 // The factorisation where every row has at most kFacMax entries up to its diagonal (2D
-// meshes), by one CTA, a dependency level at a time, a warp per row.  The general kernel
+// meshes) and levels are narrow (fac_one_cta), by one CTA, a dependency level at a time, a warp per row.  The general kernel
 // above pays, per level, the flag round trip through L2 and a gather whose places are
 // searched for: 25 us.  Here the places are found once per system (k_ilu_struct), the
 // entries of a warp's next row are on their way while it eliminates the current one, and
@@ -415,8 +415,8 @@ __global__ void __launch_bounds__(128) k_ilu_upper(int N, const int *__restrict_
 }
 
 
-// ILUPrecond of a level whose vector fits one CTA's shared memory: both triangular solves in
-// one launch of one CTA, dependency level after dependency level.  What bounds a solve is
+// ILUPrecond of a level whose vector fits one CTA's shared memory and whose dependency levels
+// are narrow (tri_one_cta): both triangular solves in one launch of one CTA, dependency level after dependency level.  What bounds a solve is
 // the round trip from a row's value to the rows that read it, once per level: 3 us through
 // L2 between warps (the kernels above).  Here a few warps solve in turn, a thread per row,
 // doing the reference's operations in the reference's order, and the values stay in shared
@@ -813,6 +813,7 @@ static int build_streams(exf_sys *s, SysLevel &L, const std::vector<int> &ptr, c
   if (sizeof(TriSmem) + (size_t)(L.N + 1) * sizeof(double) > kTriSmem) return EXF_OK;
   EXF_CUDA(cudaFuncSetAttribute(k_ilu_tri, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTriSmem));
   const TriStream T = build_tri_stream(ptr, col, dp);
+  if (!tri_one_cta(T.nrec, T.depth)) return EXF_OK;
   EXF_TRY(L.ilu_str.alloc(T.str.size()));
   EXF_TRY(L.ilu_src.alloc(T.src.size()));
   EXF_TRY(L.ilu_chunk.alloc(T.chunk.size()));
@@ -861,7 +862,7 @@ int ilu_ready(exf_sys *s, int lev) {
     EXF_CUDA(cudaMemcpyAsync(L.ilu_ord_up.p, up.data(), N * sizeof(int), cudaMemcpyHostToDevice, s->stream));
     EXF_CUDA(cudaStreamSynchronize(s->stream));
     EXF_TRY(build_streams(s, L, ptr, col, dp));
-    if (m <= kFacMax && N <= (1 << 18)) {
+    if (m <= kFacMax && N <= (1 << 18) && fac_one_cta(N, L.ilu_depth[0])) {
       std::vector<int> off(L.ilu_depth[0] + 1, 0);
       for (int i = 0; i < N; i++) off[lv[i] + 1]++;
       for (int l = 0; l < L.ilu_depth[0]; l++) off[l + 1] += off[l];

@@ -24,6 +24,7 @@ struct TriStream {
   std::vector<TriPair> src;    // {double of the stream, entry of the factor or ~row of 1 / d}
   std::vector<TriPair> chunk;  // {first word, words}
   int nrec[2] = {0, 0};        // records of the lower, the upper solve
+  int depth[2] = {0, 0};       // their dependency levels
   uint32_t first[kTriWarps] = {0};  // places of the first records, from chunk 0
 };
 
@@ -71,7 +72,7 @@ inline TriStream build_tri_stream(const std::vector<int> &ptr, const std::vector
   std::vector<TriPair> rec;  // {chunk, first word}
   for (int up = 0; up < 2; up++) {
     std::vector<int> ord, lv;
-    level_order(ptr, col, dp, up == 1, ord, &lv);
+    T.depth[up] = level_order(ptr, col, dp, up == 1, ord, &lv);
     auto len = [&](int i) { return up ? ptr[i + 1] - 1 - dp[i] : dp[i] - ptr[i]; };
     for (int a = 0; a < N;) {
       int e = a;
@@ -117,5 +118,20 @@ inline TriStream build_tri_stream(const std::vector<int> &ptr, const std::vector
   }
   return T;
 }
+
+// One CTA solves record after record, 0.31 us each; the kernels on all SMs pay a round trip
+// through L2 per dependency level, 3.0 us in 2D and 5 to 6.4 us in 3D.  ILUPrecond, one CTA
+// and all SMs (us): level-nested numbering 65 x 65 nodes (442 records, 390 levels) 138 and
+// 1172, 129 x 129 (1379, 774) 415 and 2339, 25^3 (2858, 582) 860 and 3735; numbered at random
+// within each nesting class, where levels are few and wide, 65 x 65 (296, 54) 97 and 190,
+// 129 x 129 (1064, 50) 336 and 185, 25^3 (2045, 240) 641 and 1221.
+inline bool tri_one_cta(const int nrec[2], const int depth[2]) {
+  return nrec[0] + nrec[1] <= 9 * (depth[0] + depth[1]);
+}
+// The factorisation (rows of at most kFacMax entries up to the diagonal): one CTA takes 3 us
+// and 0.2 us per row of a level's 32-row rounds, all SMs 25 us per level.  Factorisation, one
+// CTA and all SMs (ms), level-nested numbering: 33 x 33 nodes (11 rows per level) 0.62 and
+// 2.4, 65 x 65 (22) 1.5 and 4.9, 129 x 129 (43) 4.5 and 9.9, 257 x 257 (86) 15.9 and 19.9.
+inline bool fac_one_cta(int N, int depth) { return N <= 100 * depth; }
 
 }  // namespace exf

@@ -30,6 +30,7 @@ int main() {
     }
   }
   const exf::TriStream T = exf::build_tri_stream(ptr, col, dp);
+  printf("%d %d %d %d ", exf::tri_one_cta(T.nrec, T.depth), exf::fac_one_cta(N, T.depth[0]), T.depth[0], T.depth[1]);
   printf("%d %d %d %d %d %d %d %d ", exf::kTriStages, exf::kTriWarps, exf::kTriWords, (int)T.str.size(),
          (int)T.src.size(), (int)T.chunk.size(), T.nrec[0], T.nrec[1]);
   for (int w = 0; w < exf::kTriWarps; w++) printf("%u ", T.first[w]);
@@ -52,13 +53,15 @@ def builder(tmp_path_factory):
         text = "%d\n" % len(rows) + "\n".join("%d %s" % (len(r), " ".join(map(str, r))) for r in rows)
         out = subprocess.run([str(d / "s")], input=text, capture_output=True, text=True, check=True).stdout.split()
         v = np.array([int(x) for x in out], np.int64)
+        cta, v = v[:4], v[4:]
         stages, warps, words, nstr, nsrc, nch, lo, up = v[:8]
         o = 8 + warps
         first = v[8:o]
         chunk, o = v[o:o + 2 * nch].reshape(nch, 2), o + 2 * nch
         src, o = v[o:o + 2 * nsrc].reshape(nsrc, 2), o + 2 * nsrc
         return dict(stages=stages, warps=warps, words=words, first=first, chunk=chunk, src=src,
-                    str=v[o:].reshape(nstr, 4).astype(np.uint32), nlo=lo, nrec=lo + up)
+                    str=v[o:].reshape(nstr, 4).astype(np.uint32), nlo=lo, nrec=lo + up, tri_cta=bool(cta[0]),
+                    fac_cta=bool(cta[1]), depth=cta[2:])
 
     return run
 
@@ -156,3 +159,14 @@ def test_replayed_records_are_the_triangular_solves(builder, name):
         y[i] = (s + (0.0 + f[dp[i]] * w[i])) * inv[i]
     assert k == t["nrec"] and v[N] == 0.0
     assert np.array_equal(v[:N], y)
+
+
+def test_wide_levels_stay_on_all_sms(builder):
+    """Narrow levels (a row depends on the one before) go to one CTA, few wide levels do not."""
+    t = builder(lattice(33, 17))
+    assert t["tri_cta"] and t["fac_cta"]
+    t = builder(lattice(129, 129, 3))
+    assert sum(t["depth"]) < 100 and t["nrec"] > 1000
+    assert not t["tri_cta"] and not t["fac_cta"]
+    t = builder(lattice(65, 65, 3))  # a third of the records a level: still the one CTA's
+    assert t["tri_cta"]
