@@ -273,8 +273,8 @@ struct SysLevel {
   int ilu_nsrc = 0, ilu_nchunk = 0, ilu_nrec[2] = {0, 0};
   uint4 ilu_first = {0u, 0u, 0u, 0u};  // places of the first records
   // levels factored by one CTA (kFacMax entries up to the diagonal, fac_one_cta): the rows of the
-  // dense blocks of the factorisation, {entry, place} (k_ilu_struct), and the level offsets
-  DBuf<int2> ilu_ent;
+  // dense blocks of the factorisation, entry and place (k_ilu_struct), and the level offsets
+  DBuf<unsigned> ilu_ent;
   DBuf<int4> ilu_row;
   DBuf<int> ilu_pos, ilu_loff;
   bool ilu_ok = false;

@@ -254,18 +254,21 @@ __global__ void __launch_bounds__(32 * NW) k_ilu_factor(int N, const int *__rest
 // searched for: 25 us.  Here the places are found once per system (k_ilu_struct), the
 // entries of a warp's next row are on their way while it eliminates the current one, and
 // a level ends with the CTA's barrier.  Same operations, same order, same bits.
-constexpr int kFacMax = 11, kFacCap = 128, kFacLd = kFacMax + 1;
+constexpr int kFacMax = 11, kFacLd = kFacMax + 1;
+constexpr int kFacCap = 128;  // places of a row: at most kFacMax^2
+static_assert(kFacMax * kFacMax <= kFacCap && kFacMax * kFacLd < 255, "a place is a byte, 255 none");
 
-// row t of the level order: {row, first entry, entries up to the diagonal, diagonal entry};
-// its kFacCap {entry, place in the dense block} and the entries (S_a, i) of the rows in S
+// row t of the level order: {row, first entry, first of its places, diagonal entry}; its
+// places, a word each: entry << 8 | place in the dense block; and the entries (S_a, i) of the
+// rows in S.  COUNT: the number of its places alone.
+template <bool COUNT>
 __global__ void k_ilu_struct(int N, const int *__restrict__ ord, const int *__restrict__ ptr,
-                             const int *__restrict__ col, const int *__restrict__ dpos, int4 *row, int2 *ent, int *pos) {
+                             const int *__restrict__ col, const int *__restrict__ dpos, int *cnt,
+                             const int *__restrict__ off, int4 *row, unsigned *ent, int *pos) {
   const int t = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (t >= N) return;
   const int i = ord[t], k0 = ptr[i], kd = dpos[i], LD = kd - k0 + 1;
-  if (lane == 0) row[t] = make_int4(i, k0, LD, kd);
   const int S = lane < LD ? col[k0 + lane] : -1;
-  int2 *out = ent + (long)t * kFacCap;
   int n = 0;
   for (int a = 0; a < LD; a++) {
     const int r = __shfl_sync(0xffffffffu, S, a), rb = ptr[r], re = ptr[r + 1];
@@ -275,28 +278,38 @@ __global__ void k_ilu_struct(int N, const int *__restrict__ ord, const int *__re
       for (int q = 0; q < LD; q++)
         if (__shfl_sync(0xffffffffu, S, q) == c) b = q;
       const unsigned m = __ballot_sync(0xffffffffu, b >= 0);
-      if (b >= 0) out[n + __popc(m & ((1u << lane) - 1u))] = make_int2(k, a * kFacLd + b);
-      if (c == i) pos[t * 16 + a] = k;
+      if constexpr (!COUNT) {
+        if (b >= 0) ent[off[t] + n + __popc(m & ((1u << lane) - 1u))] = (unsigned)k << 8 | (unsigned)(a * kFacLd + b);
+        if (c == i) pos[t * 16 + a] = k;
+      }
       n += __popc(m);
     }
   }
-  for (int q = n + lane; q < kFacCap; q += 32) out[q] = make_int2(-1, 0);
+  if (lane > 0) return;
+  if constexpr (COUNT) {
+    cnt[t] = n;
+  } else {
+    row[t] = make_int4(i, k0, off[t], kd);
+    if (t == N - 1) row[N] = make_int4(0, 0, off[N], 0);
+  }
 }
 
 __global__ void __launch_bounds__(1024) k_ilu_factor_cta(int nlev, const int *__restrict__ loff,
-                                                         const int4 *__restrict__ row, const int2 *__restrict__ ent,
+                                                         const int4 *__restrict__ row, const unsigned *__restrict__ ent,
                                                          const int *__restrict__ pos, double *f, double *invd, int *ctl) {
   __shared__ double s_blk[32][kFacMax * kFacLd + 4];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double *B = s_blk[warp];
   int4 rw = make_int4(0, 0, 0, 0);
-  int2 e[4];
+  constexpr unsigned kNone = 0xffffffffu;
+  unsigned e[kFacCap / 32];
   int pi = 0;
   auto fetch = [&](int t) {
     rw = row[t];
+    const int n = row[t + 1].z - rw.z;
     pi = lane < 16 ? pos[t * 16 + lane] : 0;
 #pragma unroll
-    for (int q = 0; q < 4; q++) e[q] = ent[(long)t * kFacCap + 32 * q + lane];
+    for (int q = 0; q < kFacCap / 32; q++) e[q] = 32 * q + lane < n ? ent[rw.z + 32 * q + lane] : kNone;
   };
   int lo = loff[0], hi = loff[1], hi2 = nlev > 1 ? loff[2] : hi;
   if (lo + warp < hi) fetch(lo + warp);
@@ -304,16 +317,16 @@ __global__ void __launch_bounds__(1024) k_ilu_factor_cta(int nlev, const int *__
     const int hi3 = l + 3 <= nlev ? loff[l + 3] : hi2;
     bool have = lo + warp < hi;
     for (int t = lo + warp; t < hi; t += 32) {
-      double g[4];
+      double g[kFacCap / 32];
 #pragma unroll
-      for (int q = 0; q < 4; q++) g[q] = e[q].x >= 0 ? f[e[q].x] : 0.;
+      for (int q = 0; q < kFacCap / 32; q++) g[q] = e[q] != kNone ? f[e[q] >> 8] : 0.;
       for (int q = lane; q < kFacMax * kFacLd; q += 32) B[q] = 0.;
       __syncwarp();
 #pragma unroll
-      for (int q = 0; q < 4; q++)
-        if (e[q].x >= 0) B[e[q].y] = g[q];
+      for (int q = 0; q < kFacCap / 32; q++)
+        if (e[q] != kNone) B[e[q] & 255u] = g[q];
       __syncwarp();
-      const int i = rw.x, k0 = rw.y, last = rw.z - 1, kd = rw.w, pk = pi;
+      const int i = rw.x, k0 = rw.y, kd = rw.w, last = kd - k0, pk = pi;
       // the warp's next row, of this level or the next
       const int tn = t + 32 < hi ? t + 32 : hi + warp;
       if (tn < (t + 32 < hi ? hi : hi2)) fetch(tn);
@@ -807,16 +820,20 @@ static int launch_factor(exf_sys *s, SysLevel &L) {
   return EXF_OK;
 }
 
-// The streams of k_ilu_tri for one level, from the pattern (fixed per system)
+// The streams of k_ilu_tri for one level, from the pattern (fixed per system); without memory
+// for them the level is solved on all SMs
 static int build_streams(exf_sys *s, SysLevel &L, const std::vector<int> &ptr, const std::vector<int> &col,
                          const std::vector<int> &dp) {
   if (sizeof(TriSmem) + (size_t)(L.N + 1) * sizeof(double) > kTriSmem) return EXF_OK;
   EXF_CUDA(cudaFuncSetAttribute(k_ilu_tri, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTriSmem));
   const TriStream T = build_tri_stream(ptr, col, dp);
   if (!tri_one_cta(T.nrec, T.depth)) return EXF_OK;
-  EXF_TRY(L.ilu_str.alloc(T.str.size()));
-  EXF_TRY(L.ilu_src.alloc(T.src.size()));
-  EXF_TRY(L.ilu_chunk.alloc(T.chunk.size()));
+  if (L.ilu_str.alloc(T.str.size()) != EXF_OK || L.ilu_src.alloc(T.src.size()) != EXF_OK ||
+      L.ilu_chunk.alloc(T.chunk.size()) != EXF_OK) {
+    L.ilu_str.release();
+    L.ilu_src.release();
+    return EXF_OK;
+  }
   EXF_CUDA(cudaMemcpyAsync(L.ilu_str.p, T.str.data(), T.str.size() * sizeof(uint4), cudaMemcpyHostToDevice, s->stream));
   EXF_CUDA(cudaMemcpyAsync(L.ilu_src.p, T.src.data(), T.src.size() * sizeof(int2), cudaMemcpyHostToDevice, s->stream));
   EXF_CUDA(cudaMemcpyAsync(L.ilu_chunk.p, T.chunk.data(), T.chunk.size() * sizeof(int2), cudaMemcpyHostToDevice,
@@ -826,6 +843,40 @@ static int build_streams(exf_sys *s, SysLevel &L, const std::vector<int> &ptr, c
   for (int u = 0; u < 2; u++) L.ilu_nrec[u] = T.nrec[u];
   L.ilu_first = make_uint4(T.first[0], T.first[1], T.first[2], T.first[3]);
   L.ilu_nsrc = (int)T.src.size();
+  return EXF_OK;
+}
+
+// The places of k_ilu_factor_cta for one level, from the pattern and the rows' dependency
+// levels (fixed per system); without memory for them the level is factored on all SMs
+static int build_places(exf_sys *s, SysLevel &L, const std::vector<int> &lv) {
+  const int N = L.N;
+  std::vector<int> loff(L.ilu_depth[0] + 1, 0), off(N + 1, 0);
+  for (int i = 0; i < N; i++) loff[lv[i] + 1]++;
+  for (int l = 0; l < L.ilu_depth[0]; l++) loff[l + 1] += loff[l];
+  DBuf<int> d_off;
+  if (d_off.alloc(N + 1) != EXF_OK) return EXF_OK;
+  const unsigned g = (unsigned)(((long)N * 32 + 255) / 256);
+  k_ilu_struct<true><<<g, 256, 0, s->stream>>>(N, L.ilu_ord_lo.p, L.qq_ptr.p, L.qq_col.p, L.diag_pos.p, d_off.p, nullptr,
+                                               nullptr, nullptr, nullptr);
+  EXF_LAUNCH_CHECK();
+  EXF_CUDA(cudaMemcpyAsync(off.data() + 1, d_off.p, N * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  EXF_CUDA(cudaStreamSynchronize(s->stream));
+  for (int t = 0; t < N; t++) off[t + 1] += off[t];
+  if (L.ilu_loff.alloc(loff.size()) != EXF_OK || L.ilu_ent.alloc(off[N]) != EXF_OK ||
+      L.ilu_pos.alloc((size_t)N * 16) != EXF_OK || L.ilu_row.alloc(N + 1) != EXF_OK) {
+    L.ilu_ent.release();
+    L.ilu_pos.release();
+    L.ilu_row.release();
+    return EXF_OK;
+  }
+  EXF_TRY(L.ilu_pos.zero(s->stream));
+  EXF_CUDA(cudaMemcpyAsync(L.ilu_loff.p, loff.data(), loff.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
+  EXF_CUDA(cudaMemcpyAsync(d_off.p, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
+  k_ilu_struct<false><<<g, 256, 0, s->stream>>>(N, L.ilu_ord_lo.p, L.qq_ptr.p, L.qq_col.p, L.diag_pos.p, nullptr,
+                                                d_off.p, L.ilu_row.p, L.ilu_ent.p, L.ilu_pos.p);
+  EXF_LAUNCH_CHECK();
+  EXF_COUNT(2);
+  EXF_CUDA(cudaStreamSynchronize(s->stream));
   return EXF_OK;
 }
 
@@ -862,22 +913,9 @@ int ilu_ready(exf_sys *s, int lev) {
     EXF_CUDA(cudaMemcpyAsync(L.ilu_ord_up.p, up.data(), N * sizeof(int), cudaMemcpyHostToDevice, s->stream));
     EXF_CUDA(cudaStreamSynchronize(s->stream));
     EXF_TRY(build_streams(s, L, ptr, col, dp));
-    if (m <= kFacMax && N <= (1 << 18) && fac_one_cta(N, L.ilu_depth[0])) {
-      std::vector<int> off(L.ilu_depth[0] + 1, 0);
-      for (int i = 0; i < N; i++) off[lv[i] + 1]++;
-      for (int l = 0; l < L.ilu_depth[0]; l++) off[l + 1] += off[l];
-      EXF_TRY(L.ilu_loff.alloc(off.size()));
-      EXF_TRY(L.ilu_ent.alloc((size_t)N * kFacCap));
-      EXF_TRY(L.ilu_pos.alloc((size_t)N * 16));
-      EXF_TRY(L.ilu_row.alloc(N));
-      EXF_TRY(L.ilu_pos.zero(s->stream));
-      EXF_CUDA(cudaMemcpyAsync(L.ilu_loff.p, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
-      EXF_CUDA(cudaStreamSynchronize(s->stream));
-      k_ilu_struct<<<(unsigned)(((long)N * 32 + 255) / 256), 256, 0, s->stream>>>(
-          N, L.ilu_ord_lo.p, L.qq_ptr.p, L.qq_col.p, L.diag_pos.p, L.ilu_row.p, L.ilu_ent.p, L.ilu_pos.p);
-      EXF_COUNT(1);
-      EXF_LAUNCH_CHECK();
-    }
+    // (entries in 24 bits, places in 8)
+    if (m <= kFacMax && N <= (1 << 18) && L.nqq < (1 << 24) - 1 && fac_one_cta(N, L.ilu_depth[0]))
+      EXF_TRY(build_places(s, L, lv));
     L.ilu_maxl = m;
     s->buf_epoch++;
   }

@@ -141,3 +141,16 @@ def test_smoother_call(gpu_lib, dim, nlev, n0, permuted, rows, m):
     # least squares here, rotations there: rounding of m <= 33 steps of a system whose
     # preconditioned condition number is below 1e3 (the mass term of 1000 bounds it)
     assert np.linalg.norm(got - want) <= 1e-11 * np.linalg.norm(want)
+
+
+def test_factorisation_memory(gpu_lib):
+    """A 257 x 257 level: factor 8.4 MB, 63 places of 4 bytes a row 16.7 MB, entries above the
+    diagonal 4.2 MB, rows, orders and flags 2.5 MB: less than 40 MB in 2 MB pages (a fixed
+    1 KB of places a row would take 86 MB)."""
+    import torch
+    t = system(2, 7, (2, 2), False)
+    c = np.ones(t.ndof(6))
+    t.coarse_solve(np.ones(t.ndof(0)))
+    free = torch.cuda.mem_get_info()[0]
+    t.ilu_apply(6, c)
+    assert c.size == 257 * 257 and free - torch.cuda.mem_get_info()[0] < 40e6
