@@ -24,11 +24,15 @@ def sources():
     return sorted(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cpp")))
 
 
+def dependencies(src):
+    """The files whose edit makes the object of src out of date: src and every header."""
+    deps = [src] + [os.path.join(CSRC, h) for h in sorted(os.listdir(CSRC)) if h.endswith((".h", ".cuh"))]
+    return deps + [os.path.join(HERE, "..", "include", "exfemus_b200.h")]
+
+
 def _compile(src, verbose):
     obj = os.path.join(BUILD, os.path.basename(src) + ".o")
-    deps = [src] + [os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith(".h")]
-    deps.append(os.path.join(HERE, "..", "include", "exfemus_b200.h"))
-    if os.path.exists(obj) and all(os.path.getmtime(obj) >= os.path.getmtime(d) for d in deps):
+    if os.path.exists(obj) and all(os.path.getmtime(obj) >= os.path.getmtime(d) for d in dependencies(src)):
         return obj
     cmd = [NVCC] + ARCH + FLAGS + ["-c", src, "-o", obj]
     if verbose:
