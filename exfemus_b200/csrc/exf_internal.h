@@ -48,6 +48,9 @@ void count_launch(int n);  // kernels launched by the library (all streams)
     }                                                                                  \
   } while (0)
 
+// bits of a system's wait flag: whose bounded wait ran out
+constexpr int kWaitBulk = 1, kWaitCluster = 2, kWaitIlu = 4, kWaitProbe = 8;
+
 #define EXF_TRY(expr)          \
   do {                         \
     int rc__ = (expr);         \
@@ -343,7 +346,7 @@ struct exf_sys {
   bool ds_move = false;                     // DS: move the mesh at each x_old update
   exf_sys *ds_x = nullptr;                  // DS: the dx system (old x displacement)
   exf::Partials red;
-  exf::DBuf<int> wait_flag;                 // set by a bounded in-kernel wait that ran out
+  exf::DBuf<int> wait_flag;                 // bits kWait*: kernels with a bounded wait that ran out
   // per level {||b_L||^2, r^2 before the last pre-smoothing sweep, r^2 before the last
   // post-smoothing sweep (coarsest: after the solve), -}: the accuracies the reference's
   // level solver reports, for the conditional correction and the reference stop test

@@ -72,7 +72,7 @@ __device__ __forceinline__ double wait_val(const double *v, int j, int *err) {
     if ((t & 255) == 255 && *(volatile int *)err) return 0.;
     __nanosleep(32);
   }
-  atomicExch(err, 1);
+  atomicOr(err, kWaitIlu);
   return 0.;
 }
 
@@ -84,7 +84,7 @@ __device__ __forceinline__ bool wait_row(const int *flag, int j, int gen, int *e
     if ((t & 255) == 255 && *(volatile int *)err) return false;
     __nanosleep(64);
   }
-  atomicExch(err, 1);
+  atomicOr(err, kWaitIlu);
   return false;
 }
 
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(32 * NW) k_ilu_factor(int N, const int *__rest
     const int i = ord[t];
     const int k0 = ptr[i], kd = dpos[i], LD = kd - k0 + 1;
     if (LD > MAXL) {  // the host sizes MAXL from the pattern: not reached
-      if (lane == 0) atomicExch(err, 1);
+      if (lane == 0) atomicOr(err, kWaitIlu);
       if (lane == 0) st_rel(flag + i, gen);
       continue;
     }
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(32 * NW) k_ilu_factor(int N, const int *__rest
       if (k < last) {
         f[k0 + k] = lk[u];
         if (Pi[k] >= 0) f[Pi[k]] = uk[u];  // entry (S_k, i) of the earlier row S_k
-        else atomicExch(err, 1);           // LASILUStructErr: the pattern is symmetric here
+        else atomicOr(err, kWaitIlu);           // LASILUStructErr: the pattern is symmetric here
       }
     }
     if (lane == 0) {
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(kTriThreads) k_ilu_tri(int N, const uint4 *__r
       if (it + 1 < nch) ch = chunk[it + 1];
     }
     if (!ok) {  // the copies already issued land before the CTA leaves
-      atomicExch(err, 1);
+      atomicOr(err, kWaitIlu);
       for (int j = max(0, it - kTriStages); j < it; j++) mbar_wait(&S.full[j % kTriStages], (j / kTriStages) & 1);
     }
   } else if (warp < kTriWarps) {
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(kTriThreads) k_ilu_tri(int N, const uint4 *__r
       ci += next >> 24;
       const int k = ci % kTriStages;
       if (good && !mbar_wait(&S.full[k], (ci / kTriStages) & 1)) {
-        atomicExch(err, 1);
+        atomicOr(err, kWaitIlu);
         good = false;
       }
       have = good;
@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(kTriThreads) k_ilu_tri(int N, const uint4 *__r
     if (warp < nrec) fetch();
     for (int k = warp, turn = warp == 0 ? -1 : 0; k < nrec; k += kTriWarps, turn++) {
       if (turn >= 0 && !mbar_wait(&S.turn[warp], turn & 1)) {  // record k - 1 is solved
-        atomicExch(err, 1);
+        atomicOr(err, kWaitIlu);
         good = have = false;  // the turns go on without further work
       }
       if (have) tri_solve(t, v, S.part, lane, k >= nlo);

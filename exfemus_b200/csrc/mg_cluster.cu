@@ -285,7 +285,7 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
             arm();
             if (S.ok && !mbar_wait(&S.bar[S.phase & 1], (S.phase >> 1) & 1)) {
               S.ok = false;  // leave by the regular path, without further waits, sends or arrivals
-              atomicExch(S.wait_flag, 1);
+              atomicOr(S.wait_flag, kWaitCluster);
             }
             S.phase++;
           }

@@ -1584,7 +1584,7 @@ __global__ void __launch_bounds__(32 * (NWC + 1), 1)
       __syncwarp();
     }
     if (!ok) {
-      if (lane == 0) atomicExch(wait_flag, 1);
+      if (lane == 0) atomicOr(wait_flag, kWaitBulk);
       // let the copies already issued land before the CTA leaves
       for (int j = max(0, it - STG); j < it; j++) mbar_wait(&S.full[j % STG], (j / STG) & 1);
     }
@@ -1618,7 +1618,7 @@ __global__ void __launch_bounds__(32 * (NWC + 1), 1)
   for (int it = 0;; it++) {
     const int s = it % STG;
     if (!mbar_wait(&S.full[s], (it / STG) & 1)) {
-      if (lane == 0) atomicExch(wait_flag, 1);
+      if (lane == 0) atomicOr(wait_flag, kWaitBulk);
       break;
     }
     const int m = S.nrow[s];
@@ -2263,7 +2263,7 @@ __global__ void k_wait_probe(int tries, int *wait_flag) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  if (threadIdx.x == 0 && !mbar_wait(&bar, 0u, tries)) atomicExch(wait_flag, 1);
+  if (threadIdx.x == 0 && !mbar_wait(&bar, 0u, tries)) atomicOr(wait_flag, kWaitProbe);
 }
 
 int wait_probe(exf_sys *s) {
@@ -2280,7 +2280,9 @@ int device_wait_status(exf_sys *s) {
   if (flag) {
     EXF_CUDA(cudaMemsetAsync(s->wait_flag.p, 0, sizeof(int), s->stream));
     EXF_CUDA(cudaStreamSynchronize(s->stream));
-    set_error("a bounded wait of the Vanka bulk row kernel ran out");
+    set_error("a bounded wait ran out in:%s%s%s%s", flag & kWaitBulk ? " the Vanka bulk row kernel" : "",
+              flag & kWaitCluster ? " the cluster V-cycle" : "", flag & kWaitIlu ? " the ILU recurrences" : "",
+              flag & kWaitProbe ? " the wait probe" : "");
     return EXF_ERR_CUDA;
   }
   return EXF_OK;
