@@ -1459,6 +1459,7 @@ int exf_time_op(exf_sys *s, int what, int lev, const exf_mg_params *p, const exf
         return EXF_ERR_ARG;
     }
   };
+  EXF_CUDA(cudaStreamSynchronize(s->stream));  // a sweep reads the matrix before its wait
   if (what == 6) {
     *avg_ms = 0.;
     return wait_probe(s);

@@ -59,12 +59,20 @@ constexpr int kWaitBulk = 1, kWaitCluster = 2, kWaitIlu = 4, kWaitProbe = 8;
 
 // Programmatic dependent launch: kernels of the multigrid chain are launched with
 // programmatic stream serialisation so the next launch is set up while the previous grid
-// drains; every such kernel starts with EXF_PDL_WAIT (griddepcontrol.wait), before its
-// first global read, so it still observes all writes of the preceding grid.  Right after
-// the wait it releases its own dependents (griddepcontrol.launch_dependents): their
-// blocks may then be scheduled onto free SM slots, where they block in their own wait
-// until this grid has completed and its writes are visible.  Launched without the
-// attribute both instructions are no-ops.
+// drains; every such kernel runs EXF_PDL_WAIT (griddepcontrol.wait) before it reads what the
+// preceding grid may write and before it writes at all.  Right after the wait it releases
+// its own dependents (griddepcontrol.launch_dependents): their blocks may then be scheduled
+// onto free SM slots, where they block in their own wait until this grid has completed and
+// its writes are visible.  Launched without the attribute both instructions are no-ops.
+//
+// The smoothers' kernels (k_gs_colour, k_vanka_rows, _solve, _patch, _tile, _stream,
+// _rows_bulk) read matrix, couplings, patch coefficients and descriptors BEFORE the wait.
+// That is safe by one rule: the launch directly before such a kernel in its stream writes
+// none of these.  (Whatever came before that launch is complete: it had waited for it.)
+// Sweeps, residuals, transfers and vector kernels keep the rule; after a kernel that writes
+// a matrix, its copies or coefficients (assembly, sync_fp32, vanka_prep, star_pack,
+// transpose) the host waits for the stream, or a copy or another kernel lies between, before
+// the first sweep.
 #define EXF_PDL_WAIT()                                                \
   do {                                                                \
     asm volatile("griddepcontrol.wait;" ::: "memory");                \

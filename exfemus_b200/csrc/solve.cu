@@ -1763,7 +1763,7 @@ __global__ void __launch_bounds__(32 * (NWC + 1), 1)
 // stages of the BULK row kernel: per colour and CTA (grid CTAs, rows split evenly), the
 // rows cut greedily into stages of at most 32 rows and capb records, {first row, first
 // record} per stage and one closing entry per CTA
-static int bulk_schedule(SysLevel &L, int grid, int capb) {
+static int bulk_schedule(SysLevel &L, int grid, int capb, cudaStream_t st) {
   const std::vector<long long> &so = L.soff_h;
   std::vector<longlong2> e;
   std::vector<int> off;
@@ -1787,8 +1787,9 @@ static int bulk_schedule(SysLevel &L, int grid, int capb) {
   }
   EXF_TRY(L.bsched.alloc(e.size()));
   EXF_TRY(L.bsched_off.alloc(off.size()));
-  EXF_CUDA(cudaMemcpy(L.bsched.p, e.data(), e.size() * sizeof(longlong2), cudaMemcpyHostToDevice));
-  EXF_CUDA(cudaMemcpy(L.bsched_off.p, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice));
+  EXF_CUDA(cudaMemcpyAsync(L.bsched.p, e.data(), e.size() * sizeof(longlong2), cudaMemcpyHostToDevice, st));
+  EXF_CUDA(cudaMemcpyAsync(L.bsched_off.p, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+  EXF_CUDA(cudaStreamSynchronize(st));  // the row kernel reads both, and the records, before its wait
   L.bsched_G = grid;
   return EXF_OK;
 }
@@ -1889,7 +1890,7 @@ static int vanka_sweep_rows(exf_sys *s, int lev, const exf_mg_params *p, T *x, c
             return EXF_ERR_STATE;
           }
           if (!L.sv.p) EXF_TRY(star_pack(s, lev));
-          EXF_TRY(bulk_schedule(L, grid, CAPB));
+          EXF_TRY(bulk_schedule(L, grid, CAPB, s->stream));
         }
         EXF_CUDA(launch_pdl(kern, dim3(grid), dim3(32 * (NWC + 1)), sizeof(SM), s->stream,
                             (const longlong2 *)L.bsched.p, (const int *)(L.bsched_off.p + L.bsched_coff[c]),
