@@ -196,13 +196,12 @@ struct Transfer {
 // rows to the row groups of `act` CTAs
 struct CluTable {
   bool ok = false;
-  int act = 1, steps = 0, exch = 0, Np = 0, entries = 0;  // CTAs, steps and exchanges of a sweep, positions,
-                                                          // most entries of a CTA (0: too many for its
-                                                          // shared memory)
+  int act = 1, steps = 0, Np = 0, entries = 0;  // CTAs, steps of a sweep, positions, most entries of a
+                                                // CTA (0: too many for its shared memory)
   const int4 *tab = nullptr;   // [act][steps][groups] {position or -1, first entry, entries (0: padding), diagonal - first}
   const int *first = nullptr;  // [act][steps][groups] first of the row's entries in the CTA's copy
   const int2 *ent = nullptr;   // [act][entries] the copy's entries: {entry of the matrix, position of its column}
-  const int2 *step = nullptr;  // {positions of the colour, 1: last step of it, 2: first step of it}
+  const int2 *step = nullptr;  // CluStep (mg_cluster_plan.h)
   const int *node = nullptr;   // [Np] node at each position, -1 padding
   const int *col = nullptr;    // [nqq] position of each entry's column
 };

@@ -44,8 +44,8 @@ static constexpr int clu_lpr(int dim) { return dim == 2 ? 8 : 16; }
 
 template <class T>
 struct CluLevel {
-  int N, Np, steps, exch, act, mat;  // nodes, padded positions, steps and exchanges of a sweep, active
-                                     // CTAs, entries of a CTA's rows in shared memory (0: not there)
+  int N, Np, steps, act, mat;  // nodes, padded positions, steps of a sweep, active CTAs, entries
+                               // of a CTA's rows in shared memory (0: not there)
   const int4 *tab;             // CluTable
   const int *first;
   const int2 *ent;
@@ -95,7 +95,7 @@ struct CluSmem {
   T *x;
   int4 *d;         // [steps][groups of the CTA]
   T *inv, *b;
-  int2 *step;      // {positions of the colour, 1: last of it in sweep order, 2: in reverse}
+  int2 *step;      // CluStep
   T *v;            // entries (mat)
   int *c;
   uint64_t *bar;   // two mbarriers: the values of a colour, alternating
@@ -209,22 +209,12 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
   // step i of a sweep is step s0 + i * dir of the tables
   const int s0 = reverse ? steps - 1 : 0, dir = reverse ? -1 : 1;
   // the warps arrive for a colour once they have sent the colour before (while its values
-  // travel), thread 0 with the colour's bytes
-  int ai = 0, left = nsw * L.exch;  // next step to look at, of all sweeps; colours to arrive for
-  unsigned aph = S.phase;
-  auto arm = [&]() {
-    if (wl > 0 || left <= 0 || !S.ok) return;
-    if (threadIdx.x > 0) {
-      mbar_arrive(&S.bar[aph & 1]);
-    } else {
-      int2 st;
-      do {
-        st = S.step[s0 + (ai++ % steps) * dir];
-      } while (!(st.y & bit));
-      mbar_arrive_tx(&S.bar[aph & 1], (unsigned)(st.x * sizeof(T)));
-    }
-    aph++;
-    left--;
+  // travel), thread 0 with the colour's bytes, which the step before it in the order holds
+  auto arrive = [&](unsigned phase, int next) {
+    if (wl > 0 || !S.ok) return;
+    const unsigned count = reverse ? (unsigned)next >> 16 : (unsigned)next & 0xffffu;
+    if (threadIdx.x > 0) mbar_arrive(&S.bar[phase & 1]);
+    else mbar_arrive_tx(&S.bar[phase & 1], count * (unsigned)sizeof(T));
   };
   const unsigned dst = (unsigned)wl / PK;  // the CTA this lane sends to, its vector
   const int hv = wl % PK;
@@ -234,7 +224,7 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
     ax = cluster_addr(S.x + hv * VL, dst);
     ab = cluster_addr(S.bar, dst);
   }
-  if (L.act > 1) arm();
+  if (L.act > 1 && total > 0) arrive(S.phase, S.step[steps - 1 - s0].x);
   RowSlot<T, E> s[PF];
   int ld = s0, nld = 0;  // table step of the next load
   auto load = [&](RowSlot<T, E> &r) {
@@ -254,7 +244,7 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
     for (int u = 0; u < PF; u++) {
       if (it + u < total) {
         const int4 q = sd[cs * GC];
-        const bool end = S.step[cs].y & bit;
+        const int2 st = S.step[cs];
         const T xn = (sb[cs * GC] - row_dot<T, LPR, E, false>(col, vv, s[u], q, lane, S.x)) * sinv[cs * GC];
         if (L.act == 1) {
           if (q.x >= 0 && lane == 0) S.x[q.x] = xn;
@@ -278,11 +268,11 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
           cs = s0;
         }
         if (it + u + PF < total) load(s[u]);
-        if (end) {
+        if (st.y & bit) {
           if (L.act == 1) {
             __syncthreads();
           } else {
-            arm();
+            if (it + u + 1 < total) arrive(S.phase + 1, st.x);
             if (S.ok && !mbar_wait(&S.bar[S.phase & 1], (S.phase >> 1) & 1)) {
               S.ok = false;  // leave by the regular path, without further waits, sends or arrivals
               atomicOr(S.wait_flag, kWaitCluster);
@@ -552,7 +542,6 @@ int cluster_ready(exf_sys *s) {
     C.act = P.act;
     C.Np = (int)P.node.size();
     C.steps = (int)P.step.size();
-    C.exch = P.exch;
     // entries that fit no CTA's shared memory are read from the level's arrays
     C.entries = (size_t)P.entries * (4 + sizeof(float)) > kCluSmem ? 0 : P.entries;
     at[l] = {put(P.tab), put(P.first), put(P.step), put(P.node), put(P.pos), 0, 0};
@@ -626,7 +615,6 @@ int mg_cluster(exf_sys *s, int hi, const exf_mg_params *p, int mul_hi) {
     if (l == 0) break;
     d.Np = L.clu.Np;
     d.steps = L.clu.steps;
-    d.exch = L.clu.exch;
     d.act = L.clu.act;
     d.mat = S.mat[l];
     d.tab = L.clu.tab;

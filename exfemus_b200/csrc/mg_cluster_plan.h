@@ -1,6 +1,7 @@
 // mg_cluster_plan.h -- which CTA, warp and step of the cluster kernel (mg_cluster.cu) updates
-// which row of a scalar level, and which levels fit one launch.  Host code on plain arrays, no CUDA types, so that the rules
-// the kernel's exchange rests on can be checked without a device.
+// which row of a scalar level, and which levels fit one launch.  Host code on plain arrays,
+// no CUDA types, so that the rules the kernel's exchange rests on can be checked without a
+// device.
 #pragma once
 #include <algorithm>
 #include <cstddef>
@@ -17,11 +18,11 @@ struct CluRow {  // a row group's row in one step
   int pos, k0, len, diag;  // position or -1 (none), first entry, entries (0: padding), diagonal - first
 };
 struct CluStep {
-  int count, flags;  // positions of the colour; 1: last step of it, 2: first step of it
+  int next, flags;  // positions of the colour after its own, of the one before << 16 (both
+                    // cyclic); 1: last step of its colour, 2: first step of it
 };
 struct CluPlan {
   int act = 1;      // CTAs that share the level
-  int exch = 0;     // colours with rows: exchanges of a sweep
   int entries = 0;  // most matrix entries of a CTA, a multiple of 4
   std::vector<int> node, pos;  // node at each position (-1 padding), position of each node
   std::vector<CluStep> step;   // steps of a sweep
@@ -30,7 +31,7 @@ struct CluPlan {
 };
 
 // qp: row pointers, diag: absolute diagonal entries, items: the nodes by colour; lpr lanes
-// per row, CTAs of nt threads, `most` CTAs in the cluster.
+// per row, CTAs of nt threads, `most` CTAs in the cluster; less than 2^15 positions.
 //
 // Positions are the nodes in colour order (a colour's rows longest first, so that a warp's
 // rows are alike, each colour padded to whole warps); a colour's units of one warp are dealt
@@ -49,7 +50,7 @@ inline CluPlan plan_cluster(int N, const int *qp, const int *diag, int ncolour, 
   P.pos.assign(N, -1);
   int longest = 0;
   for (int i = 0; i < N; i++) longest = std::max(longest, qp[i + 1] - qp[i]);
-  std::vector<int> cbase(ncolour), rounds(ncolour), units(ncolour), at(longest + 1);
+  std::vector<int> cbase(ncolour), rounds(ncolour), units(ncolour), at(longest + 1), used;
   for (int c = 0; c < ncolour; c++) {
     const int n = col_off[c + 1] - col_off[c];
     units[c] = (n + rw - 1) / rw;
@@ -70,9 +71,12 @@ inline CluPlan plan_cluster(int N, const int *qp, const int *diag, int ncolour, 
       P.pos[*v] = p;
     }
     rounds[c] = (units[c] + P.act * nw - 1) / (P.act * nw);
-    for (int k = 0; k < rounds[c]; k++)
-      P.step.push_back({units[c] * rw, (k == rounds[c] - 1 ? 1 : 0) | (k == 0 ? 2 : 0)});
-    P.exch += n > 0;
+    if (rounds[c] > 0) used.push_back(c);
+  }
+  for (size_t k = 0; k < used.size(); k++) {
+    const int c = used[k], after = used[(k + 1) % used.size()], before = used[(k + used.size() - 1) % used.size()];
+    for (int r = 0; r < rounds[c]; r++)
+      P.step.push_back({units[after] * rw | units[before] * rw << 16, (r == rounds[c] - 1 ? 1 : 0) | (r == 0 ? 2 : 0)});
   }
   const int steps = (int)P.step.size();
   P.tab.assign((size_t)P.act * steps * gc, CluRow{-1, 0, 0, -1});

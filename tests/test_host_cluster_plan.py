@@ -30,10 +30,10 @@ int main() {
   std::vector<int> at(off.begin(), off.end() - 1);
   for (int i = 0; i < N; i++) items[at[col[i]]++] = i;
   const exf::CluPlan P = exf::plan_cluster(N, qp.data(), diag.data(), nc, off.data(), items.data(), lpr, nt, most);
-  printf("%d %d %d %d %d\n", P.act, P.exch, P.entries, (int)P.node.size(), (int)P.step.size());
+  printf("%d %d %d %d\n", P.act, P.entries, (int)P.node.size(), (int)P.step.size());
   for (int v : P.node) printf("%d ", v);
   for (int v : P.pos) printf("%d ", v);
-  for (auto &s : P.step) printf("%d %d ", s.count, s.flags);
+  for (auto &s : P.step) printf("%d %d ", s.next, s.flags);
   for (size_t q = 0; q < P.tab.size(); q++)
     printf("%d %d %d %d %d ", P.tab[q].pos, P.tab[q].k0, P.tab[q].len, P.tab[q].diag, P.first[q]);
 }
@@ -58,13 +58,13 @@ def planner(tmp_path_factory):
         text += "\n".join("%d %d" % cl for cl in zip(colour, length))
         out = subprocess.run([str(d / "plan")], input=text, capture_output=True, text=True, check=True).stdout.split()
         v = np.array([int(x) for x in out])
-        act, exch, entries, npos, steps = v[:5]
-        o = 5
+        act, entries, npos, steps = v[:4]
+        o = 4
         node, o = v[o:o + npos], o + npos
         pos, o = v[o:o + colour.size], o + colour.size
         step, o = v[o:o + 2 * steps].reshape(steps, 2), o + 2 * steps
         tab = v[o:].reshape(act, steps, NT // lpr, 5)
-        return dict(act=act, exch=exch, entries=entries, node=node, pos=pos, step=step, tab=tab, rw=32 // lpr,
+        return dict(act=act, entries=entries, node=node, pos=pos, step=step, tab=tab, rw=32 // lpr,
                     nw=NT // 32)
 
     return run
@@ -123,12 +123,13 @@ def test_plan(planner, name):
     # a warp's groups hold consecutive positions from a multiple of the vector's length
     lead = tab[:, :, ::rw, 0]
     assert np.all((lead < 0) | (lead % rw == 0))
-    # a step's colour, its byte count, and the same count sent by all CTAs together
+    # a step names the values that all CTAs together send in the colours around its own
     col_of_step = np.cumsum((p["step"][:, 1] & 2) > 0) - 1
     u = units(p)
-    assert p["exch"] == len(u) == len(np.unique(colour)) == ((p["step"][:, 1] & 1) > 0).sum()
+    assert len(u) == len(np.unique(colour)) == ((p["step"][:, 1] & 1) > 0).sum()
     for c in range(len(u)):
-        assert np.all(p["step"][col_of_step == c, 0] == u[c].sum())
+        assert np.all(p["step"][col_of_step == c, 0] & 0xffff == u[(c + 1) % len(u)].sum())
+        assert np.all(p["step"][col_of_step == c, 0] >> 16 == u[c - 1].sum())
     if p["act"] > 1:
         assert np.all(u.sum(axis=2) > 0), "a CTA sends nothing in a colour"
 
