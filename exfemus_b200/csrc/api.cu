@@ -219,6 +219,11 @@ float *lvr<float>(SysLevel &L) { return L.r32.p; }
 // correction and for the reference stop test
 static bool needs_acc(const exf_mg_params *p) { return p->cond_corr || p->stop_test == EXF_STOP_REFERENCE; }
 
+// whether a cycle of these parameters may run in the cluster kernel
+static bool cluster_cycle(const exf_mg_params *p) {
+  return p->smoother == EXF_SMOOTH_GS && p->gamma == 1 && !needs_acc(p);
+}
+
 // One smoothing call of nsw sweeps.  With acc, it also leaves in *slot the squared
 // residual that the reference's level solver reports as its accuracy: LASPACK's
 // stationary iterations evaluate ||r||/||b|| on a residual refreshed only while
@@ -260,8 +265,7 @@ static int mg_step(exf_sys *s, int lev, const exf_mg_params *p, bool final_resid
   }
   const int mul = (p->double_below_top && lev < top) ? 2 : 1;
   // Gauss-Seidel levels that fit a cluster: this level and all below it in one launch
-  if (p->smoother == EXF_SMOOTH_GS && p->gamma == 1 && !acc &&
-      mg_cluster_level(s, lev, sizeof(T), (p->nu_pre + p->nu_post) * mul)) {
+  if (cluster_cycle(p) && mg_cluster_level(s, lev, sizeof(T), (p->nu_pre + p->nu_post) * mul)) {
     if (!s->coarse_ok) EXF_TRY(coarse_factor(s));
     EXF_TRY(mg_cluster<T>(s, lev, p, mul));
     if (final_resid) EXF_TRY(spmv_resid<T>(s, lev, x, b, r, d_norm_out));
@@ -1223,7 +1227,7 @@ int exf_mg_solve(exf_sys *s, const exf_mg_params *p, exf_solve_stats *st) {
     }
     for (int l = p->coarse_iters > 0 ? 0 : 1; l < s->nlev; l++) EXF_TRY(ilu_ready(s, l));  // once per assembly
   }
-  if (p->smoother == EXF_SMOOTH_GS) EXF_TRY(cluster_ready(s));
+  if (cluster_cycle(p)) EXF_TRY(cluster_ready(s));
   if (!s->coarse_ok) EXF_TRY(coarse_factor(s));
   EXF_CUDA(cudaEventRecord(s->ev0, s->stream));
   EXF_TRY(norm2(s, T.b.p, T.ndof, dnb));
@@ -1419,7 +1423,7 @@ int exf_time_op(exf_sys *s, int what, int lev, const exf_mg_params *p, const exf
   if (what == 2 && !ph) return EXF_ERR_ARG;
   if (what != 2 && !s->assembled) return EXF_ERR_STATE;
   if (what == 3) EXF_TRY(need_transfers(s));
-  if (what == 3 && p->smoother == EXF_SMOOTH_GS) EXF_TRY(cluster_ready(s));
+  if (what == 3 && cluster_cycle(p)) EXF_TRY(cluster_ready(s));
   if (!s->coarse_ok && what == 3) EXF_TRY(coarse_factor(s));
   SysLevel &L = s->L[lev];
   const bool f32 = p->precision == EXF_PREC_MIXED;
