@@ -193,6 +193,8 @@ __device__ __forceinline__ void store_x(const CluLevel<T> &L, int gt, int nth, c
 //    padding if need be), hence after phase p of every CTA: its bytes cannot count as colour
 //    p's, nor can it overwrite a value that a warp still reads for colour p + 1 (that warp
 //    has not sent yet).
+// A warp whose wait runs out leaves the sweep; so do, each after its own limit, the warps that
+// wait for it (a flag looked at before every send and arrival instead: 4% of a V-cycle).
 // Entries that are not in shared memory (!MAT) are loaded two or three steps ahead.
 template <class T, int LPR, int E, bool MAT>
 __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int reverse, CluSmem<T> &S) {
@@ -211,7 +213,7 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
   // the warps arrive for a colour once they have sent the colour before (while its values
   // travel), thread 0 with the colour's bytes, which the step before it in the order holds
   auto arrive = [&](unsigned phase, int next) {
-    if (wl > 0 || !S.ok) return;
+    if (wl > 0) return;
     const unsigned count = reverse ? (unsigned)next >> 16 : (unsigned)next & 0xffffu;
     if (threadIdx.x > 0) mbar_arrive(&S.bar[phase & 1]);
     else mbar_arrive_tx(&S.bar[phase & 1], count * (unsigned)sizeof(T));
@@ -255,10 +257,10 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
             const T v0 = __shfl_sync(0xffffffffu, xn, (hv * VL) * LPR);
             const T v1 = __shfl_sync(0xffffffffu, xn, (hv * VL + 1) * LPR);
             if constexpr (VL == 2) {
-              if (sender && S.ok) cluster_send2(at, v0, v1, bar);
+              if (sender) cluster_send2(at, v0, v1, bar);
             } else {
               const T v2 = __shfl_sync(0xffffffffu, xn, 2 * LPR), v3 = __shfl_sync(0xffffffffu, xn, 3 * LPR);
-              if (sender && S.ok) cluster_send4(at, v0, v1, v2, v3, bar);
+              if (sender) cluster_send4(at, v0, v1, v2, v3, bar);
             }
           }
         }
@@ -273,9 +275,10 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
             __syncthreads();
           } else {
             if (it + u + 1 < total) arrive(S.phase + 1, st.x);
-            if (S.ok && !mbar_wait(&S.bar[S.phase & 1], (S.phase >> 1) & 1)) {
-              S.ok = false;  // leave by the regular path, without further waits, sends or arrivals
+            if (!__all_sync(0xffffffffu, mbar_wait(&S.bar[S.phase & 1], (S.phase >> 1) & 1))) {
+              S.ok = false;  // the warp sends and arrives no more, here and on the other shared levels
               atomicOr(S.wait_flag, kWaitCluster);
+              return;
             }
             S.phase++;
           }
@@ -287,6 +290,7 @@ __device__ __forceinline__ void sweep_level(const CluLevel<T> &L, int nsw, int r
 
 template <class T, int LPR, int E>
 __device__ __forceinline__ void sweeps(const CluLevel<T> &L, int nsw, int reverse, CluSmem<T> &S) {
+  if (L.act > 1 && !S.ok) return;  // (a level of one CTA has no waits but the CTA's barriers)
   if (L.mat) sweep_level<T, LPR, E, true>(L, nsw, reverse, S);
   else sweep_level<T, LPR, E, false>(L, nsw, reverse, S);
 }
