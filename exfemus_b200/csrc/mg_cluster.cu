@@ -35,8 +35,8 @@ static constexpr int kCluNT = 512;
 // Rows of the coarsest level up to which its product runs in the cluster.  It reads n^2
 // doubles through at most 16 SMs; above, the descent and the ascent are two launches around
 // the product on all SMs.  Two-level V-cycle with one pre- and post-sweep, in one launch and
-// in three (FP64, us): n = 289 39 and 41, 625 43 and 42, 729 (3D) 102 and 102, 1225 56 and
-// 52, 2401 113 and 78, 4761 645 and 172 (FP32 9801: 2186 and 429).
+// in three (FP64, us): n = 289 37 and 39, 625 42 and 41, 729 (3D) 92 and 92, 1225 56 and 52,
+// 2401 113 and 80, 4761 629 and 168.
 static constexpr int kCluCoarse = 700;
 // lanes per row; a warp's rows are consecutive in colour order, so their new values leave
 // as vectors

@@ -113,12 +113,12 @@ inline CluPlan plan_cluster(int N, const int *qp, const int *diag, int ncolour, 
 // `sweeps` sweeps per cycle.  A sweep in the cluster grows with the rows (16 SMs) while
 // launches cost the same up to here, and the restriction, prolongation and residual that go
 // with the level lose from the start.  V-cycle down from such a level, cluster and launches
-// (us): 2D FP64 9,409 rows 2 sweeps 125 and 127, 12,769 rows 2 sweeps 137 and 129, 4 sweeps
-// 191 and 195, 16,641 rows 8 sweeps 336 and 332, 12 sweeps 456 and 465; FP32 16,641 rows 4
-// sweeps 187 and 178, 8 sweeps 279 and 293, 25,921 rows 12 sweeps 474 and 417; 6,561 rows 1
-// sweep 91 and 94, 0 sweeps 73 and 64.  3D FP32 18,785 rows 2 sweeps 245 and 242, 25,625 rows
-// 4 sweeps 393 and 406, 30,625 rows 8 sweeps 792 and 732; FP64 18,785 rows 1 sweep 207 and
-// 200, 2 sweeps 285 and 308.
+// (us): 2D FP64 9,409 rows 2 sweeps 122 and 120, 12,769 rows 2 sweeps 135 and 124, 4 sweeps
+// 188 and 187, 16,641 rows 8 sweeps 329 and 320, 12 sweeps 446 and 447; FP32 12,769 rows 4
+// sweeps 163 and 166, 16,641 rows 4 sweeps 177 and 170, 8 sweeps 261 and 277, 25,921 rows 12
+// sweeps 446 and 396; 6,561 rows 1 sweep 91 and 93, 0 sweeps 73 and 64.  3D FP32 18,785 rows 2
+// sweeps 230 and 231, 25,625 rows 2 sweeps 247 and 239, 4 sweeps 373 and 394, 30,625 rows 8
+// sweeps 733 and 707; FP64 18,785 rows 1 sweep 195 and 201, 2 sweeps 264 and 298.
 constexpr int cluster_rows(int dim, int sweeps) {
   return sweeps < 1    ? 0
          : dim == 3    ? 26000 - 14000 / sweeps
