@@ -15,7 +15,7 @@
 // phase (1,200 of them the release), 8-byte stores to 16 CTAs 2,000 (the packets bound it:
 // hence colour order and vectors), descriptors read from global memory in the phase +500.
 // V-cycle of the 32 x 32 conduction workload (4 levels, 180 phases): 0.45 -> 0.17 ms; of a
-// 128 x 64 scalar system (6 levels, the four below the top here) 0.63 -> 0.38 ms.
+// 128 x 64 scalar system (6 levels, the four below the top here) 0.63 -> 0.37 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
