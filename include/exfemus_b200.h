@@ -120,7 +120,7 @@ typedef struct {
   int double_below_top;/* 1: sweeps doubled below the top level (MGStep)           */
   int smoother;        /* EXF_SMOOTH_*                                             */
   double omega;        /* Vanka damping                                            */
-  double corr_damp;    /* coarse-correction factor (reference 0.95)                */
+  double corr_damp;    /* coarse-correction factor (reference 0.95); 0: x = P x_c  */
   int cond_corr;       /* 1: reference's conditional coarse correction: x += 0.95 P x_c */
                        /* only when the coarse accuracy is below the pre-smoothing one */
                        /* (src/MGSolverBase.C:262-263)                                 */
